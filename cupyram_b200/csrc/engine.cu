@@ -52,6 +52,7 @@
 
 #include "../../include/cupyram_b200.h"
 #include "march_col.cuh"
+#include "march_reg.cuh"
 #include "march_common.cuh"
 #include "march_sum.cuh"
 #include "pade.h"
@@ -625,7 +626,8 @@ struct cr_engine {
     // column-parallel march: rays marched by one thread-block cluster each,
     // one launch per (Pade term count) group on its own stream
     struct ColGroup {
-        int cluster, terms, nz_max, begin, count;
+        int cluster, terms, rows, nz_max, begin, count;  // rows: of a lane (march_reg.cu), 0: march_col.cu
+        bool policy;                                     // rays that the column policy took
         cudaStream_t stream;
         cudaEvent_t done;
     };
@@ -1270,6 +1272,83 @@ std::vector<char> pick_column_rays(const cr_batch* b, const std::vector<int>& pd
     return col;
 }
 
+// Clusters of march_reg.cu resident at once, by (device, cluster, terms, rows,
+// grids), asked of the driver once per process.
+std::mutex g_reg_mu;
+std::map<std::tuple<int, int, int, int, int>, int> g_reg_active;
+int reg_active(int device, int cluster, int terms, int rows, int grids) {
+    const auto key = std::make_tuple(device, cluster, terms, rows, grids ? 1 : 0);
+    std::lock_guard<std::mutex> lock(g_reg_mu);
+    auto it = g_reg_active.find(key);
+    if (it == g_reg_active.end())
+        it = g_reg_active.emplace(key, crk::reg_max_active_clusters(cluster, terms, rows, 32 * rows * cluster, grids)).first;
+    return it->second;
+}
+
+// Microseconds of one step of march_reg.cu with `rows` rows a lane, with the
+// SMs' other CTAs at work.  B200, np 6: 2.3 / 2.7 / 3.1 / 3.5 / 4.9 us at 4 / 6 /
+// 8 / 10 / 12 rows on single CTAs; 0.5 us more on pairs, 0.8 us more on
+// clusters of 16 (the exchange).
+double reg_step_us(int cluster, int rows) {
+    const double t = 1.55 + 0.19 * rows + (rows > 10 ? 1.0 : 0.0);
+    return cluster == 1 ? t : t + 0.4 + 0.1 * std::log2((double)cluster);
+}
+
+// Cluster and rows of a lane of the rays that march_reg.cu takes: in complex128,
+// every ray whose column fits the registers of at most 16 CTAs.  Against the
+// batched kernel (72-78e9 term-rows per second at any depth, bound by its
+// streams from memory) it marched 123e9 on one CTA of 380 rows, 107e9 on two,
+// 104e9 at 2300 and 3800 rows and 78e9 at 5700 rows (16 CTAs of 12 rows a lane).
+//
+// The cluster of a ray is the one that minimises the larger of its own march
+// and the whole batch's at that shape's throughput: long rays of an uneven
+// batch get many CTAs and short steps, the others few and full lanes.  Up to
+// nine rays have the GPU to themselves: they get what march_col.cu would give
+// them (as many CTAs as there are SMs, at least 64 rows each).
+struct RegPlan {
+    int cluster = 0, rows = 0;
+};
+std::vector<RegPlan> plan_reg(const cr_batch* b, const std::vector<int>& pd_n, int device) {
+    std::vector<RegPlan> plan((size_t)b->n_rays);
+    const char* env = getenv("CUPYRAM_B200_COL");
+    if ((env && env[0] == '0') || g_in_tuner) return plan;
+    if (b->precision != CR_PLAIN_C128 && b->precision != CR_C64_REFINED) return plan;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    double total = 0.0;  // term-rows of the batch
+    for (int i = 0; i < b->n_rays; ++i)
+        total += (double)b->rays[i].nz * (b->rays[i].nr + 3) * col_terms(pd_n, i);
+    std::map<std::tuple<int, int, int>, RegPlan> known;  // by nz, terms, steps
+    for (int i = 0; i < b->n_rays; ++i) {
+        const int nz = b->rays[i].nz, terms = col_terms(pd_n, i), steps = b->rays[i].nr + 3;
+        const auto key = std::make_tuple(nz, terms, steps);
+        auto it = known.find(key);
+        if (it == known.end()) {
+            RegPlan best;
+            double best_us = INFINITY;
+            const int alone = std::min({16, sms / b->n_rays, std::max(1, nz / 64)});
+            for (int C = 1; C <= 16; ++C) {
+                const int rows = crk::reg_rows(nz, C);
+                if (!rows || (C > 1 && nz < 64 * C)) continue;
+                if (b->n_rays <= 9 && C < alone) continue;
+                const int active = reg_active(device, C, terms, rows, b->compute_grids);
+                if (active <= 0) continue;
+                const double us = reg_step_us(C, rows);
+                const double all = total * us / ((double)nz * terms * active), own = steps * us;
+                const double t = std::max(all, own) + 1e-3 * all;
+                if (t < best_us) {
+                    best_us = t;
+                    best = RegPlan{C, rows};
+                }
+                if (b->n_rays <= 9) break;
+            }
+            it = known.emplace(key, best).first;
+        }
+        plan[(size_t)i] = it->second;
+    }
+    return plan;
+}
+
 }  // namespace
 
 int cr_create(const cr_batch* b, cr_engine** out) {
@@ -1335,6 +1414,10 @@ int cr_create(const cr_batch* b, cr_engine** out) {
     if (e->sum_mode) {
         MarchCosts costs;
         const std::vector<char> is_col = pick_column_rays(b, e->pd_n, b->precision, e->device, &costs);
+        const std::vector<RegPlan> reg = plan_reg(b, e->pd_n, e->device);
+        int n_policy = 0;  // rays that the column policy took
+        for (char c : is_col) n_policy += c;
+        e->st.column_rays = n_policy;
         e->st.tuner_row_step_s = costs.row_step_s;
         e->st.tuner_updates_per_s = costs.updates_per_s;
         e->st.tuner_slots = costs.slots;
@@ -1342,7 +1425,7 @@ int cr_create(const cr_batch* b, cr_engine** out) {
         // floor(32/G) rays of G lanes each, G = the largest np in the tile
         std::vector<int> bord;
         for (int rid : order)
-            if (!is_col[(size_t)rid]) bord.push_back(rid);
+            if (!is_col[(size_t)rid] && reg[(size_t)rid].rows == 0) bord.push_back(rid);
         // A tile marches in lockstep for its deepest ray's rows and its
         // longest ray's steps, so its rays should agree in both: within a
         // lane count G, rays are sorted by steps, and runs of 16 tiles'
@@ -1416,14 +1499,23 @@ int cr_create(const cr_batch* b, cr_engine** out) {
         // first; their ray columns are packed 32 to a tile after the batched ones
         std::vector<int> cord;
         for (int rid : order)
-            if (is_col[(size_t)rid]) cord.push_back(rid);
+            if (is_col[(size_t)rid] || reg[(size_t)rid].rows > 0) cord.push_back(rid);
         auto terms_of = [&](int rid) { return col_terms(e->pd_n, rid); };
         const bool chosen = b->precision == CR_CHOSEN_C64R || b->precision == CR_CHOSEN_C64;
-        const std::vector<int> csize = column_clusters(b, e->pd_n, is_col, chosen);
+        std::vector<int> csize = column_clusters(b, e->pd_n, is_col, chosen);
+        std::vector<int> lrows((size_t)b->n_rays, 0);
+        for (int rid : cord)
+            if (reg[(size_t)rid].rows > 0) {
+                csize[(size_t)rid] = reg[(size_t)rid].cluster;
+                lrows[(size_t)rid] = reg[(size_t)rid].rows;
+            }
         std::stable_sort(cord.begin(), cord.end(), [&](int x, int y) {
             const int tx = terms_of(x), ty = terms_of(y);
+            if (is_col[(size_t)x] != is_col[(size_t)y]) return is_col[(size_t)x] > is_col[(size_t)y];
             if (tx != ty) return tx > ty;
+            if (lrows[(size_t)x] != lrows[(size_t)y]) return lrows[(size_t)x] > lrows[(size_t)y];
             if (csize[(size_t)x] != csize[(size_t)y]) return csize[(size_t)x] > csize[(size_t)y];
+            if (lrows[(size_t)x] && b->rays[x].nr != b->rays[y].nr) return b->rays[x].nr > b->rays[y].nr;
             return b->rays[x].nz > b->rays[y].nz;
         });
         for (size_t q = 0; q < cord.size(); q += kTile) {
@@ -1445,12 +1537,27 @@ int cr_create(const cr_batch* b, cr_engine** out) {
         for (size_t q = 0; q < cord.size();) {
             size_t end = q;
             const int terms = terms_of(cord[q]);
-            const int nz_max = b->rays[cord[q]].nz;
-            const int cluster = csize[(size_t)cord[q]];
-            while (end < cord.size() && terms_of(cord[end]) == terms && csize[(size_t)cord[end]] == cluster) ++end;
-            e->col_groups.push_back({cluster, terms, nz_max, (int)q, (int)(end - q), nullptr, nullptr});
+            const int cluster = csize[(size_t)cord[q]], rows = lrows[(size_t)cord[q]];
+            const char policy = is_col[(size_t)cord[q]];
+            int nz_max = 0;
+            while (end < cord.size() && is_col[(size_t)cord[end]] == policy && terms_of(cord[end]) == terms && csize[(size_t)cord[end]] == cluster &&
+                   lrows[(size_t)cord[end]] == rows)
+                nz_max = std::max(nz_max, b->rays[cord[end++]].nz);
+            e->col_groups.push_back({cluster, terms, rows, nz_max, (int)q, (int)(end - q), policy != 0, nullptr, nullptr});
             q = end;
         }
+        // the groups with the longest marches are launched first
+        std::vector<double> longest(e->col_groups.size(), 0.0);
+        std::vector<size_t> turn(e->col_groups.size());
+        std::iota(turn.begin(), turn.end(), (size_t)0);
+        for (size_t q = 0; q < e->col_groups.size(); ++q)
+            for (int k = e->col_groups[q].begin; k < e->col_groups[q].begin + e->col_groups[q].count; ++k)
+                longest[q] = std::max(longest[q], (double)b->rays[cord[k]].nr *
+                                                      (e->col_groups[q].rows ? 1.0 + 0.1 * e->col_groups[q].rows : 4.0));
+        std::stable_sort(turn.begin(), turn.end(), [&](size_t x, size_t y) { return longest[x] > longest[y]; });
+        std::vector<cr_engine::ColGroup> ordered;
+        for (size_t q : turn) ordered.push_back(e->col_groups[q]);
+        e->col_groups.swap(ordered);
         for (const auto& g : e->col_groups)
             for (int k = g.begin; k < g.begin + g.count; ++k) e->term_capacity[(size_t)cord[k]] = g.terms;
         e->col_ray = cord;
@@ -1601,7 +1708,6 @@ int cr_create(const cr_batch* b, cr_engine** out) {
     e->st.tile_rays = kTile;
     e->st.n_tiles = e->n_tiles;
     e->st.device_bytes = e->device_bytes;
-    e->st.column_rays = (int)e->col_ray.size();
     e->st.create_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_create).count();
     *out = e;
     return CR_OK;
@@ -1755,7 +1861,7 @@ int cr_march(cr_engine* e) {
         ca.compute_grids = e->compute_grids;
         const int chosen = e->precision == CR_CHOSEN_C64R || e->precision == CR_CHOSEN_C64;
         ce = cudaEventRecord(e->ev[0], e->stream);
-        int nl = 0;
+        int nl = 0, n_policy = 0;
         // column groups first, each on its own stream (they hold the longest
         // marches), then the batched tiles on the engine's stream
         if (ce == cudaSuccess) ce = cudaEventRecord(e->ev_fork, e->stream);
@@ -1765,9 +1871,12 @@ int cr_march(cr_engine* e) {
             if (ce == cudaSuccess) ce = cudaStreamWaitEvent(g.stream, e->ev_fork, 0);
             crk::ColArgs ga = ca;
             ga.col_ray = e->d_col_ray + g.begin;
-            if (ce == cudaSuccess) ce = crk::launch_march_col(ga, g.count, g.cluster, g.terms, g.nz_max, chosen, g.stream);
+            if (ce == cudaSuccess) ce = 
+                    g.rows ? crk::launch_march_reg(ga, g.count, g.cluster, g.terms, g.rows, g.nz_max, g.stream)
+                           : crk::launch_march_col(ga, g.count, g.cluster, g.terms, g.nz_max, chosen, g.stream);
             if (ce == cudaSuccess) ce = cudaEventRecord(g.done, g.stream);
             ++nl;
+            n_policy += g.policy ? 1 : 0;
         }
         sa.tile_begin = 0;
         sa.ticket = e->d_ticket;
@@ -1802,7 +1911,7 @@ int cr_march(cr_engine* e) {
         for (auto& g : e->col_groups)
             if (ce == cudaSuccess) ce = cudaStreamWaitEvent(e->stream, g.done, 0);
         e->st.kernel_launches = nl + nb;
-        e->st.column_launches = nl;
+        e->st.column_launches = n_policy;
     } else if (ce == cudaSuccess) {
         ce = cudaEventRecord(e->ev[0], e->stream);
         if (ce == cudaSuccess) {
