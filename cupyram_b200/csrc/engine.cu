@@ -56,6 +56,7 @@
 #include "march_common.cuh"
 #include "march_sum.cuh"
 #include "pade.h"
+#include "pade_warp.cuh"
 
 namespace {
 
@@ -842,21 +843,28 @@ struct PadeJob {
     int np, ns, ip, pad_;
 };
 
-// One thread per job: the FP64 Pade construction of pade.h on the device.
-// pd1 / pd2 get CR_MAX_NP coefficients per job (zeros past np); status gets
-// CR_OK, CR_EPADE (Laguerre did not converge) or CR_EINVAL.
-__global__ void pade_batch_kernel(const PadeJob* __restrict__ jobs, int n, double2* __restrict__ pd1,
-                                  double2* __restrict__ pd2, int* __restrict__ status) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per job: the FP64 construction of pade.h on the device (pade_warp.cuh).
+// pd1 / pd2 get CR_MAX_NP coefficients per job (zeros past np, and for a job
+// that fails); status gets CR_OK, CR_EPADE (Laguerre did not converge) or
+// CR_EINVAL.
+constexpr int kPadeWarps = 2;  // jobs of a block: few, so that few jobs spread over many SMs
+__global__ void __launch_bounds__(32 * kPadeWarps) pade_batch_kernel(const PadeJob* __restrict__ jobs, int n,
+                                                                     double2* __restrict__ pd1,
+                                                                     double2* __restrict__ pd2,
+                                                                     int* __restrict__ status) {
+    __shared__ cr::PadeShared S[kPadeWarps];
+    __shared__ cr::cd out[kPadeWarps][2][CR_MAX_NP];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * kPadeWarps + w;
     if (i >= n) return;
     const PadeJob j = jobs[i];
-    cr::cd a[CR_MAX_NP], c[CR_MAX_NP];
-    const int rc = cr::pade_coefficients(j.freq, j.c0, j.np, j.ns, j.dr, j.ip, a, c);
-    status[i] = rc == cr::kPadeOk ? CR_OK : (rc == cr::kPadeNoConverge ? CR_EPADE : CR_EINVAL);
-    for (int k = 0; k < CR_MAX_NP; ++k) {
-        const bool on = rc == cr::kPadeOk && k < j.np;
-        pd1[(size_t)i * CR_MAX_NP + k] = on ? make_double2(a[k].re, a[k].im) : make_double2(0.0, 0.0);
-        pd2[(size_t)i * CR_MAX_NP + k] = on ? make_double2(c[k].re, c[k].im) : make_double2(0.0, 0.0);
+    const int rc = cr::pade_warp(S[w], j.freq, j.c0, j.np, j.ns, j.dr, j.ip, out[w][0], out[w][1]);
+    __syncwarp();
+    if (lane == 0) status[i] = rc == cr::kPadeOk ? CR_OK : (rc == cr::kPadeNoConverge ? CR_EPADE : CR_EINVAL);
+    if (lane < CR_MAX_NP) {
+        const bool on = rc == cr::kPadeOk && lane < j.np;
+        const cr::cd a = out[w][0][lane], c = out[w][1][lane];
+        pd1[(size_t)i * CR_MAX_NP + lane] = on ? make_double2(a.re, a.im) : make_double2(0.0, 0.0);
+        pd2[(size_t)i * CR_MAX_NP + lane] = on ? make_double2(c.re, c.im) : make_double2(0.0, 0.0);
     }
 }
 
@@ -878,7 +886,13 @@ cudaError_t device_pade(const std::vector<PadeJob>& jobs, std::vector<double2>& 
     const size_t bj = r256(jobs.size() * sizeof(PadeJob)), bp = r256(pd1.size() * sizeof(double2)),
                  bs = r256((size_t)n * sizeof(int));
     unsigned char* d = nullptr;
-    ce = cudaMallocAsync((void**)&d, bj + 2 * bp + bs, st);
+    // from the engines' pool, which keeps its memory (the default pool maps and
+    // unmaps it on every call)
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    ce = cudaGetDevice(&dev);
+    if (ce == cudaSuccess) ce = engine_pool(dev, &pool);
+    if (ce == cudaSuccess) ce = cudaMallocFromPoolAsync((void**)&d, bj + 2 * bp + bs, pool, st);
     if (ce == cudaSuccess) {
         PadeJob* dj = (PadeJob*)d;
         double2* d1 = (double2*)(d + bj);
@@ -886,9 +900,7 @@ cudaError_t device_pade(const std::vector<PadeJob>& jobs, std::vector<double2>& 
         int* ds = (int*)(d + bj + 2 * bp);
         ce = cudaMemcpyAsync(dj, jobs.data(), jobs.size() * sizeof(PadeJob), cudaMemcpyHostToDevice, st);
         if (ce == cudaSuccess) {
-            // 32 threads a block: the solves are long serial chains, so the
-            // jobs are spread over as many SMs as possible
-            pade_batch_kernel<<<(n + 31) / 32, 32, 0, st>>>(dj, n, d1, d2, ds);
+            pade_batch_kernel<<<(n + kPadeWarps - 1) / kPadeWarps, 32 * kPadeWarps, 0, st>>>(dj, n, d1, d2, ds);
             ce = cudaGetLastError();
         }
         const size_t np2 = pd1.size() * sizeof(double2);
