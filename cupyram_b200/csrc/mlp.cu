@@ -516,6 +516,232 @@ __global__ void __launch_bounds__(kUThreads) gemm_tn_tma(const __grid_constant__
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(UBN));
 }
 
+// ---------------------------------------------------------------------------
+// The default: gemm_tn_tma's loads and MMAs on blocks of 128 x BN, and an
+// epilogue that leaves by the tensor memory accelerator too.
+//
+// The surrogate's contractions range from 512 x 512 to 8192 x 8192.  A block
+// of 256 columns leaves a 512 x 512 product to 8 CTAs that each write 128 KB;
+// blocks of 64 columns spread it over 32, with eight stages in flight (22 ->
+// 9 us at K = 512).  The epilogue takes 32 (f32) or 64 (bf16) columns of a
+// warp's 32 rows at a time from tensor memory, applies bias, ReLU or mask in
+// registers, writes them to shared memory in the swizzle of the output's
+// tensor map (conflict-free 16-byte stores, a row per lane) and stores the
+// piece with one bulk copy while the next is prepared; the mask block came in
+// by bulk copies during the main loop.  Element by element the sums over K are
+// the MMAs' own, in the same order for every BN.
+// ---------------------------------------------------------------------------
+template <int EPI>
+constexpr bool epi_bf16() { return EPI == CR_MLP_EPI_BIAS_RELU_BF16 || EPI == CR_MLP_EPI_RELU_MASK_BF16; }
+template <int EPI, int BN, int ST>
+struct TileGemm {
+    static constexpr int kStage = kUTileA + BN * UBK * 2;
+    static constexpr int kMask = EPI == CR_MLP_EPI_RELU_MASK_BF16 ? UBM * BN * 2 : 0;
+    static constexpr size_t smem = (size_t)ST * kStage + kMask + BN * sizeof(float) + 1024 + 256;
+    static_assert(ST * kStage >= 4 * 8192, "the output pieces reuse the stages");
+};
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(x), "r"(y), "r"(smem_u32(src))
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// 32 consecutive columns of this lane's row of the accumulator
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, float* v) {
+    uint32_t u[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
+        "%29,%30,%31}, [%32];"
+        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
+          "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]),
+          "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]),
+          "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(u[j]);
+}
+
+template <int EPI, int BN, int ST>
+__global__ void __launch_bounds__(kUThreads)
+    gemm_tn_tile(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                 const __grid_constant__ CUtensorMap mapO, const __grid_constant__ CUtensorMap mapM, int K,
+                 const float* __restrict__ bias, int* err) {
+    using T = TileGemm<EPI, BN, ST>;
+    constexpr bool kMasked = EPI == CR_MLP_EPI_RELU_MASK_BF16;
+    constexpr bool kBias = EPI == CR_MLP_EPI_BIAS_RELU_BF16 || EPI == CR_MLP_EPI_BIAS_F32;
+    constexpr uint32_t idesc =
+        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(UBM >> 4) << 24);
+    extern __shared__ __align__(1024) unsigned char usmem[];
+    unsigned char* base = (unsigned char*)(((uintptr_t)usmem + 1023) & ~(uintptr_t)1023);
+    auto tA = [&](int st) { return base + st * T::kStage; };
+    auto tB = [&](int st) { return base + st * T::kStage + kUTileA; };
+    unsigned char* masks = base + ST * T::kStage;  // [BN / 64] blocks of 128 rows x 64 columns
+    float* sbias = (float*)(masks + T::kMask);  // the block's bias values
+    uint64_t* full = (uint64_t*)(sbias + BN);
+    uint64_t* empty = full + ST;
+    uint64_t* done = empty + ST;
+    uint64_t* mask_bar = done + 1;
+    uint32_t* taddr_s = (uint32_t*)(mask_bar + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int bm = blockIdx.y * UBM, bn = blockIdx.x * BN;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(taddr_s)),
+                     "r"(BN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    if (tid == 32) {
+        for (int s = 0; s < ST; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(done, 1);
+        mbar_init(mask_bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (kBias)
+        for (int c = tid; c < BN; c += kUThreads) sbias[c] = bias[bn + c];
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *taddr_s;
+    const int nk = K / UBK;
+    bool ok = true;
+
+    int issued = 0;  // producer: tiles whose loads were issued
+    if (warp == 0 && lane == 0) {
+        for (int kt = 0; kt < nk && ok; ++kt) {
+            const int st = kt % ST;
+            if (kt >= ST) ok &= mbar_wait(&empty[st], ((kt / ST) - 1) & 1);
+            if (!ok) break;
+            mbar_expect_tx(&full[st], (unsigned)T::kStage);
+            tma_load_2d(tA(st), &mapA, kt * UBK, bm, &full[st]);
+            tma_load_2d(tB(st), &mapB, kt * UBK, bn, &full[st]);
+            issued = kt + 1;
+            if (kMasked && kt == 0) {
+                mbar_expect_tx(mask_bar, (unsigned)T::kMask);
+#pragma unroll 1
+                for (int c = 0; c < BN / 64; ++c) tma_load_2d(masks + c * UBM * 128, &mapM, bn + 64 * c, bm, mask_bar);
+            }
+        }
+    } else if (warp == 1 && lane == 0) {
+        for (int kt = 0; kt < nk && ok; ++kt) {
+            const int st = kt % ST;
+            ok &= mbar_wait(&full[st], (kt / ST) & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t sa = smem_u32(tA(st)), sb = smem_u32(tB(st));
+#pragma unroll
+            for (int k = 0; k < UBK / 16; ++k) {
+                const uint64_t da = umma_desc_sw128(sa + k * 32), db = umma_desc_sw128(sb + k * 32);
+                const uint32_t acc = (kt > 0 || k > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "setp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                    :
+                    : "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc)
+                    : "memory");
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_u32(&empty[st]))
+                         : "memory");
+        }
+        // the accumulator is complete once every MMA issued so far is
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_u32(done))
+                     : "memory");
+    }
+    __syncwarp();
+    ok &= mbar_wait(done, 0);
+    if (kMasked) ok &= mbar_wait(mask_bar, 0);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // a role thread that gave up is seen by the whole CTA
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    if (!ok && warp == 0 && lane == 0) {
+        // no copy may still be writing this CTA's shared memory when it exits:
+        // wait (bounded) for the last load issued into each stage
+        for (int kt = issued - 1; kt >= 0 && kt >= issued - ST; --kt) mbar_wait(&full[kt % ST], (kt / ST) & 1);
+        if (kMasked && issued > 0) mbar_wait(mask_bar, 0);
+    }
+    if (!ok) {
+        if (tid == 0) atomicExch(err, 1);
+    } else {
+        constexpr int kCols = epi_bf16<EPI>() ? 64 : 32;  // columns of a piece: 128 bytes a row
+        unsigned char* stg = base + warp * 8192;           // two pieces of 4 KB; the stages are idle now
+        const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16);
+        const int row = warp * 32 + lane;
+#pragma unroll 1
+        for (int c = 0; c < BN / kCols; ++c) {
+            uint32_t w[32];  // the lane's 128 bytes
+#pragma unroll
+            for (int h = 0; h < kCols / 32; ++h) {
+                float v[32];
+                tmem_ld32(acc + (uint32_t)(c * kCols + 32 * h), v);
+                if (kBias) {
+                    const float4* b4 = reinterpret_cast<const float4*>(sbias + c * kCols + 32 * h);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float4 b = b4[j];
+                        v[4 * j] += b.x;
+                        v[4 * j + 1] += b.y;
+                        v[4 * j + 2] += b.z;
+                        v[4 * j + 3] += b.w;
+                    }
+                }
+                if (EPI == CR_MLP_EPI_BIAS_RELU_BF16) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
+                }
+                if (kMasked) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int ch = 4 * h + j;
+                        const uint4 m = *reinterpret_cast<const uint4*>(masks + c * UBM * 128 + row * 128 +
+                                                                       ((ch ^ (row & 7)) << 4));
+                        const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mm[q]));
+                            v[8 * j + 2 * q] = f.x > 0.f ? v[8 * j + 2 * q] : 0.f;
+                            v[8 * j + 2 * q + 1] = f.y > 0.f ? v[8 * j + 2 * q + 1] : 0.f;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    if (!epi_bf16<EPI>()) {
+                        w[j] = __float_as_uint(v[j]);
+                    } else if ((j & 1) == 0) {
+                        const __nv_bfloat162 p = __floats2bfloat162_rn(v[j], v[j + 1]);
+                        w[16 * h + j / 2] = *reinterpret_cast<const uint32_t*>(&p);
+                    }
+                }
+            }
+            unsigned char* piece = stg + (c & 1) * 4096;
+            if (c >= 2) {  // the copy that read this piece two turns ago is done with it
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                __syncwarp();
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<uint4*>(piece + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                    make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tma_store_2d(&mapO, bn + c * kCols, bm + warp * 32, piece);
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
+}
+
 // dst[c][r] = src[r][c] for a rows x cols BF16 matrix (32 x 32 tiles).
 __global__ void transpose_bf16(const __nv_bfloat16* __restrict__ src, int lds, __nv_bfloat16* __restrict__ dst,
                                int ldd, int rows, int cols) {
@@ -532,30 +758,115 @@ __global__ void transpose_bf16(const __nv_bfloat16* __restrict__ src, int lds, _
     }
 }
 
-// out[c] = sum_r src[r][c] (bias gradients), one thread per column.
-__global__ void col_sum_bf16(const __nv_bfloat16* __restrict__ src, int ld, int rows, int cols, float* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.f;
-    for (int r = 0; r < rows; ++r) s += __bfloat162float(src[(size_t)r * ld + c]);
-    out[c] = s;
+// Several matrices of one launch (the layers of a network).
+constexpr int kMaxMats = 32;
+struct Mats {
+    int n;
+    int first[kMaxMats + 1];  // first block of each matrix
+    const __nv_bfloat16* src[kMaxMats];
+    void* dst[kMaxMats];
+    int lds[kMaxMats], ldd[kMaxMats], rows[kMaxMats], cols[kMaxMats];
+};
+__device__ __forceinline__ int mat_of(const Mats& t, int block) {
+    int i = 0;
+    while (block >= t.first[i + 1]) ++i;
+    return i;
+}
+
+// dst[c][r] = src[r][c] in 64 x 64 tiles: 16-byte rows in and out (columns and
+// rows multiples of 64, bases and strides 16-byte aligned).  All layers of a
+// training step in one launch, instead of twelve of 3.5-11 us.
+__global__ void __launch_bounds__(256) transpose_mats(const __grid_constant__ Mats t) {
+    __shared__ __nv_bfloat16 tile[64][72];
+    const int i = mat_of(t, blockIdx.x), b = blockIdx.x - t.first[i], nc = t.cols[i] / 64;
+    const int r0 = (b / nc) * 64, c0 = (b % nc) * 64;
+    const __nv_bfloat16* src = t.src[i];
+    __nv_bfloat16* dst = (__nv_bfloat16*)t.dst[i];
+    for (int q = threadIdx.x; q < 512; q += 256) {
+        const int r = q >> 3, c = (q & 7) * 8;
+        const uint4 v = *reinterpret_cast<const uint4*>(src + (size_t)(r0 + r) * t.lds[i] + c0 + c);
+        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tile[c + j][r] = e[j];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 512; q += 256) {
+        const int c = q >> 3, r = (q & 7) * 8;
+        *reinterpret_cast<uint4*>(dst + (size_t)(c0 + c) * t.ldd[i] + r0 + r) =
+            *reinterpret_cast<const uint4*>(&tile[c][r]);
+    }
+}
+
+// out[c] = sum_r src[r][c] (bias gradients): a block takes 64 columns, 32 of
+// its rows of threads every 32nd row, folded in a fixed order.  One thread a
+// column waited for 512 loads in turn (32-37 us a layer).
+__global__ void __launch_bounds__(1024) col_sum_mats(const __grid_constant__ Mats t) {
+    __shared__ float2 part[32][33];
+    const int i = mat_of(t, blockIdx.x), c = (blockIdx.x - t.first[i]) * 64 + 2 * threadIdx.x;
+    const __nv_bfloat16* src = t.src[i];
+    const bool pair = c + 1 < t.cols[i] && (((uintptr_t)src & 3) == 0) && t.lds[i] % 2 == 0;
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int r = threadIdx.y; r < t.rows[i]; r += 32) {
+        const __nv_bfloat16* q = src + (size_t)r * t.lds[i] + c;
+        if (pair) {
+            const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(q));
+            s.x += v.x;
+            s.y += v.y;
+        } else {
+            if (c < t.cols[i]) s.x += __bfloat162float(q[0]);
+            if (c + 1 < t.cols[i]) s.y += __bfloat162float(q[1]);
+        }
+    }
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    for (int d = 16; d > 0; d >>= 1) {
+        if ((int)threadIdx.y < d) {
+            const float2 o = part[threadIdx.y + d][threadIdx.x];
+            part[threadIdx.y][threadIdx.x].x += o.x;
+            part[threadIdx.y][threadIdx.x].y += o.y;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.y == 0) {
+        float* out = (float*)t.dst[i];
+        if (c < t.cols[i]) out[c] = part[0][threadIdx.x].x;
+        if (c + 1 < t.cols[i]) out[c + 1] = part[0][threadIdx.x].y;
+    }
 }
 
 // Masked mean squared error: grad = 2 (pred - y) / n_valid where valid,
 // and the sum of squared errors accumulated into *sse.
+__device__ __forceinline__ float mse_one(float pred, float y, bool valid, float inv_count, double& acc) {
+    if (!valid) return 0.f;
+    const float d = pred - y;
+    acc += (double)d * d;
+    return 2.f * d * inv_count;
+}
+// VEC: four entries a thread at a time (n a multiple of 4, aligned arrays).
+template <bool VEC>
 __global__ void mse_grad(const float* __restrict__ pred, const __nv_bfloat16* __restrict__ y,
                          const unsigned char* __restrict__ valid, long long n, float inv_count,
                          __nv_bfloat16* __restrict__ grad, double* __restrict__ sse) {
     __shared__ double red[256];
     double acc = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        float g = 0.f;
-        if (valid[i]) {
-            const float d = pred[i] - __bfloat162float(y[i]);
-            g = 2.f * d * inv_count;
-            acc += (double)d * d;
+    const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    if (VEC) {
+        for (long long i = first; i < n / 4; i += stride) {
+            const float4 p = reinterpret_cast<const float4*>(pred)[i];
+            const uint2 yb = reinterpret_cast<const uint2*>(y)[i];
+            const uchar4 ok = reinterpret_cast<const uchar4*>(valid)[i];
+            const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&yb.x)),
+                         y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&yb.y));
+            const float g0 = mse_one(p.x, y0.x, ok.x, inv_count, acc), g1 = mse_one(p.y, y0.y, ok.y, inv_count, acc),
+                        g2 = mse_one(p.z, y1.x, ok.z, inv_count, acc), g3 = mse_one(p.w, y1.y, ok.w, inv_count, acc);
+            const __nv_bfloat162 a = __floats2bfloat162_rn(g0, g1), b = __floats2bfloat162_rn(g2, g3);
+            reinterpret_cast<uint2*>(grad)[i] =
+                make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
         }
-        grad[i] = __float2bfloat16_rn(g);
+    } else {
+        for (long long i = first; i < n; i += stride)
+            grad[i] = __float2bfloat16_rn(mse_one(pred[i], __bfloat162float(y[i]), valid[i], inv_count, acc));
     }
     red[threadIdx.x] = acc;
     __syncthreads();
@@ -567,18 +878,140 @@ __global__ void mse_grad(const float* __restrict__ pred, const __nv_bfloat16* __
 }
 
 // Adam on FP32 master parameters; writes the BF16 copy used by the GEMMs.
+struct AdamArgs {
+    float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ float adam_one(float p, float g, float& m, float& v, const AdamArgs& a, float wd) {
+    const float gi = g + wd * p;
+    m = a.b1 * m + (1.f - a.b1) * gi;
+    v = a.b2 * v + (1.f - a.b2) * gi * gi;
+    return p - a.lr * (m * a.c1) / (sqrtf(v * a.c2) + a.eps);
+}
 __global__ void adam_step(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                          float* __restrict__ v, __nv_bfloat16* __restrict__ pb, long long n, float lr, float b1,
-                          float b2, float eps, float c1, float c2, float wd) {
+                          float* __restrict__ v, __nv_bfloat16* __restrict__ pb, long long n, AdamArgs a, float wd) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float gi = g[i] + wd * p[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+        float mi = m[i], vi = v[i];
+        const float pi = adam_one(p[i], g[i], mi, vi, a, wd);
         m[i] = mi;
         v[i] = vi;
-        const float pi = p[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
         p[i] = pi;
         if (pb) pb[i] = __float2bfloat16_rn(pi);
+    }
+}
+
+// The same over every layer's weights and biases in one launch, writing the
+// weights' BF16 copy and its transpose too (64 x 64 tiles): bound by the 32
+// bytes a parameter that it moves.  Eight Adam launches and four transposes
+// read the weights twice.
+struct AdamMats {
+    int n;
+    int first[kMaxMats + 1];  // first block: weights in 64 x 64 tiles, biases in runs of 4096
+    float* p[kMaxMats];
+    const float* g[kMaxMats];
+    float *m[kMaxMats], *v[kMaxMats];
+    __nv_bfloat16 *pb[kMaxMats], *pt[kMaxMats];  // NULL: a bias
+    int rows[kMaxMats], cols[kMaxMats];
+};
+__global__ void __launch_bounds__(256) adam_mats(const __grid_constant__ AdamMats t, AdamArgs a, float wd) {
+    __shared__ __nv_bfloat16 tile[64][72];
+    int i = 0;
+    while ((int)blockIdx.x >= t.first[i + 1]) ++i;
+    const int b = blockIdx.x - t.first[i];
+    if (!t.pb[i]) {
+        const int n = t.rows[i];
+        for (int q = b * 4096 + threadIdx.x; q < min(n, (b + 1) * 4096); q += 256) {
+            float m = t.m[i][q], v = t.v[i][q];
+            t.p[i][q] = adam_one(t.p[i][q], t.g[i][q], m, v, a, 0.f);
+            t.m[i][q] = m;
+            t.v[i][q] = v;
+        }
+        return;
+    }
+    const int nc = t.cols[i] / 64, r0 = (b / nc) * 64, c0 = (b % nc) * 64;
+#pragma unroll 2
+    for (int q = threadIdx.x; q < 1024; q += 256) {
+        const int r = q >> 4, c = (q & 15) * 4;
+        const size_t o = (size_t)(r0 + r) * t.cols[i] + c0 + c;
+        float4 p = *reinterpret_cast<const float4*>(t.p[i] + o), m = *reinterpret_cast<const float4*>(t.m[i] + o),
+               v = *reinterpret_cast<const float4*>(t.v[i] + o);
+        const float4 g = *reinterpret_cast<const float4*>(t.g[i] + o);
+        p.x = adam_one(p.x, g.x, m.x, v.x, a, wd);
+        p.y = adam_one(p.y, g.y, m.y, v.y, a, wd);
+        p.z = adam_one(p.z, g.z, m.z, v.z, a, wd);
+        p.w = adam_one(p.w, g.w, m.w, v.w, a, wd);
+        *reinterpret_cast<float4*>(t.p[i] + o) = p;
+        *reinterpret_cast<float4*>(t.m[i] + o) = m;
+        *reinterpret_cast<float4*>(t.v[i] + o) = v;
+        __nv_bfloat162 w[2] = {__floats2bfloat162_rn(p.x, p.y), __floats2bfloat162_rn(p.z, p.w)};
+        *reinterpret_cast<uint2*>(t.pb[i] + o) = *reinterpret_cast<const uint2*>(w);
+        tile[c][r] = w[0].x;
+        tile[c + 1][r] = w[0].y;
+        tile[c + 2][r] = w[1].x;
+        tile[c + 3][r] = w[1].y;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 512; q += 256) {
+        const int c = q >> 3, r = (q & 7) * 8;
+        *reinterpret_cast<uint4*>(t.pt[i] + (size_t)(c0 + c) * t.rows[i] + r0 + r) =
+            *reinterpret_cast<const uint4*>(&tile[c][r]);
+    }
+}
+
+// Mean and standard deviation (over the members) of the ensemble's outputs,
+// each scaled, shifted and clamped: one pass over the members' outputs
+// instead of a stack, three elementwise passes and two reductions over it.
+constexpr int kMaxMembers = 64;
+struct Members {
+    const float* out[kMaxMembers];
+};
+__device__ __forceinline__ float member_tl(float x, float scale, float mid, float lo, float hi) {
+    const float t = __fadd_rn(__fmul_rn(x, scale), mid);
+    return t < lo ? lo : (t > hi ? hi : t);  // a NaN stays
+}
+template <int M>  // members held in registers; 0: any number, read twice
+__global__ void __launch_bounds__(256) ensemble_stats(const __grid_constant__ Members p, int members, long long n4,
+                                                      float scale, float mid, float lo, float hi,
+                                                      float4* __restrict__ mean, float4* __restrict__ spread) {
+    const float inv = 1.f / (float)members;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+        auto get = [&](int k) {
+            float4 x = __ldcs(reinterpret_cast<const float4*>(p.out[k]) + i);
+            x.x = member_tl(x.x, scale, mid, lo, hi);
+            x.y = member_tl(x.y, scale, mid, lo, hi);
+            x.z = member_tl(x.z, scale, mid, lo, hi);
+            x.w = member_tl(x.w, scale, mid, lo, hi);
+            return x;
+        };
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f), q = s, x[M > 0 ? M : 1];
+        auto add = [&](const float4& v) {
+            s.x += v.x;
+            s.y += v.y;
+            s.z += v.z;
+            s.w += v.w;
+        };
+        auto dev = [&](const float4& v) {
+            q.x = fmaf(v.x - s.x, v.x - s.x, q.x);
+            q.y = fmaf(v.y - s.y, v.y - s.y, q.y);
+            q.z = fmaf(v.z - s.z, v.z - s.z, q.z);
+            q.w = fmaf(v.w - s.w, v.w - s.w, q.w);
+        };
+        if (M > 0) {
+#pragma unroll
+            for (int k = 0; k < M; ++k) x[k] = get(k);
+#pragma unroll
+            for (int k = 0; k < M; ++k) add(x[k]);
+        } else {
+            for (int k = 0; k < members; ++k) add(get(k));
+        }
+        s = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
+        if (M > 0) {
+#pragma unroll
+            for (int k = 0; k < M; ++k) dev(x[k]);
+        } else {
+            for (int k = 0; k < members; ++k) dev(get(k));
+        }
+        mean[i] = s;
+        spread[i] = make_float4(sqrtf(q.x * inv), sqrtf(q.y * inv), sqrtf(q.z * inv), sqrtf(q.w * inv));
     }
 }
 
@@ -788,6 +1221,56 @@ bool operand_map(CUtensorMap* map, const void* ptr, int rows, int K, int ld, int
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tensor map of a rows x cols output (f32 or bf16) or mask in boxes of 128
+// bytes x box_rows rows, 128-byte swizzle.
+bool tile_map(CUtensorMap* map, const void* ptr, bool bf16, int rows, int cols, int ld, int box_rows) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    const int eb = bf16 ? 2 : 4;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * eb};
+    const cuuint32_t box[2] = {(cuuint32_t)(128 / eb), (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    return enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+               const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+struct TileOperands {
+    const void *A, *B;
+    int M, N, K, lda, ldb;
+};
+
+template <int EPI, int BN, int ST>
+cudaError_t launch_tile(const TileOperands& o, const EpiArgs& e, int* err, cudaStream_t st) {
+    using T = TileGemm<EPI, BN, ST>;
+    CUtensorMap ma, mb, mo, mm;
+    if (!operand_map(&ma, o.A, o.M, o.K, o.lda, UBM) || !operand_map(&mb, o.B, o.N, o.K, o.ldb, BN) ||
+        !tile_map(&mo, e.out, epi_bf16<EPI>(), o.M, o.N, e.ldo, 32))
+        return cudaErrorUnknown;
+    mm = mo;
+    if (T::kMask && !tile_map(&mm, e.mask, true, o.M, o.N, e.ldm, UBM)) return cudaErrorUnknown;
+    const cudaError_t ce = cudaFuncSetAttribute(gemm_tn_tile<EPI, BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)T::smem);
+    if (ce != cudaSuccess) return ce;
+    gemm_tn_tile<EPI, BN, ST><<<dim3(o.N / BN, o.M / UBM), kUThreads, T::smem, st>>>(ma, mb, mo, mm, o.K, e.bias, err);
+    return cudaGetLastError();
+}
+
+// The widest block that still gives every SM of the device work (148 on a
+// B200; two blocks each at 256 columns, whose two CTAs share an SM).
+template <int EPI>
+cudaError_t launch_tile_n(const TileOperands& o, const EpiArgs& e, int* err, cudaStream_t st) {
+    constexpr int kSms = 148;
+    const long long rows = o.M / UBM;
+    if constexpr (EPI != CR_MLP_EPI_RELU_MASK_BF16) {
+        if (rows * (o.N / 256) >= 2 * kSms) return launch_tile<EPI, 256, 2>(o, e, err, st);
+    }
+    if (rows * (o.N / 128) >= kSms) return launch_tile<EPI, 128, 3>(o, e, err, st);
+    return launch_tile<EPI, 64, 7>(o, e, err, st);
+}
+
 }  // namespace
 
 extern "C" {
@@ -855,6 +1338,20 @@ int cr_mlp_gemm_tc(int epi, const void* A, const void* B, int M, int N, int K, i
         if (ce != cudaSuccess) return CR_MLP_ECUDA;
         return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
     }
+    // outputs (and a mask) whose rows start on 16-byte boundaries leave by bulk copies
+    const bool half = epi == CR_MLP_EPI_BIAS_RELU_BF16 || epi == CR_MLP_EPI_RELU_MASK_BF16;
+    const bool out16 = aligned16(out) && ldo % (half ? 8 : 4) == 0;
+    if (feed == 1 && out16 && (epi != CR_MLP_EPI_RELU_MASK_BF16 || (aligned16(mask) && ldm % 8 == 0))) {
+        const TileOperands o{A, B, M, N, K, lda, ldb};
+        switch (epi) {
+            case CR_MLP_EPI_BIAS_RELU_BF16: ce = launch_tile_n<CR_MLP_EPI_BIAS_RELU_BF16>(o, e, err, st); break;
+            case CR_MLP_EPI_BIAS_F32: ce = launch_tile_n<CR_MLP_EPI_BIAS_F32>(o, e, err, st); break;
+            case CR_MLP_EPI_F32: ce = launch_tile_n<CR_MLP_EPI_F32>(o, e, err, st); break;
+            case CR_MLP_EPI_RELU_MASK_BF16: ce = launch_tile_n<CR_MLP_EPI_RELU_MASK_BF16>(o, e, err, st); break;
+            default: return CR_MLP_EBADSHAPE;
+        }
+        return ce == cudaSuccess ? 0 : CR_MLP_ECUDA;
+    }
     if (feed == 1) {
         // operands by the tensor memory accelerator (tensor maps over this GPU's memory)
         CUtensorMap ma, mb;
@@ -902,25 +1399,179 @@ int cr_mlp_transpose(const void* src, int lds, void* dst, int ldd, int rows, int
 
 int cr_mlp_col_sum(const void* src, int ld, int rows, int cols, float* out, void* stream) {
     if (rows <= 0 || cols <= 0 || ld < cols) return CR_MLP_EBADSHAPE;
-    col_sum_bf16<<<(cols + 255) / 256, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)src, ld, rows, cols, out);
+    Mats t{};
+    t.n = 1;
+    t.first[1] = (cols + 63) / 64;
+    t.src[0] = (const __nv_bfloat16*)src;
+    t.dst[0] = out;
+    t.lds[0] = ld;
+    t.rows[0] = rows;
+    t.cols[0] = cols;
+    col_sum_mats<<<t.first[1], dim3(32, 32), 0, (cudaStream_t)stream>>>(t);
     return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
 }
 
 int cr_mlp_mse_grad(const float* pred, const void* target, const unsigned char* valid, long long n, float inv_count,
                     void* grad, double* sse, void* stream) {
     if (n <= 0) return CR_MLP_EBADSHAPE;
-    mse_grad<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(pred, (const __nv_bfloat16*)target, valid, n, inv_count,
-                                                            (__nv_bfloat16*)grad, sse);
+    const bool vec = n % 4 == 0 && aligned16(pred) && ((uintptr_t)target & 7) == 0 && ((uintptr_t)grad & 7) == 0 &&
+                     ((uintptr_t)valid & 3) == 0;
+    cudaStream_t st = (cudaStream_t)stream;
+    auto y = (const __nv_bfloat16*)target;
+    auto gr = (__nv_bfloat16*)grad;
+    // four blocks an SM: each block's sum of squares is one atomic
+    const long long want = ((vec ? n / 4 : n) + 255) / 256;
+    const int grid = (int)(want < 592 ? want : 592);
+    if (vec) mse_grad<true><<<grid, 256, 0, st>>>(pred, y, valid, n, inv_count, gr, sse);
+    else mse_grad<false><<<grid, 256, 0, st>>>(pred, y, valid, n, inv_count, gr, sse);
     return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
+}
+
+static AdamArgs adam_args(float lr, float beta1, float beta2, float eps, int step) {
+    return AdamArgs{lr, beta1, beta2, eps, 1.f / (1.f - powf(beta1, (float)step)),
+                    1.f / (1.f - powf(beta2, (float)step))};
 }
 
 int cr_mlp_adam(float* p, const float* g, float* m, float* v, void* p_bf16, long long n, float lr, float beta1,
                 float beta2, float eps, int step, float weight_decay, void* stream) {
     if (n <= 0 || step < 1) return CR_MLP_EBADSHAPE;
-    const float c1 = 1.f / (1.f - powf(beta1, (float)step));
-    const float c2 = 1.f / (1.f - powf(beta2, (float)step));
-    adam_step<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(p, g, m, v, (__nv_bfloat16*)p_bf16, n, lr, beta1, beta2,
-                                                             eps, c1, c2, weight_decay);
+    adam_step<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(p, g, m, v, (__nv_bfloat16*)p_bf16, n,
+                                                             adam_args(lr, beta1, beta2, eps, step), weight_decay);
+    return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
+}
+
+namespace {
+int mlp_gemm_any(int epi, int tc, const void* A, const void* B, int M, int N, int K, int lda, int ldb, void* out,
+                 const float* bias, const void* mask, int ldm, int* err, void* stream) {
+    if (tc && N % UBN == 0 && K % UBK == 0)
+        return cr_mlp_gemm_tc(epi, A, B, M, N, K, lda, ldb, out, N, bias, mask, ldm, err, stream);
+    return cr_mlp_gemm(epi, A, B, M, N, K, lda, ldb, out, N, bias, mask, ldm, stream);
+}
+bool mlp_dims_ok(const cr_mlp_net* net, int batch) {
+    if (!net || net->layers < 1 || batch <= 0 || batch % 128) return false;
+    for (int l = 0; l <= net->layers; ++l)
+        if (net->dims[l] <= 0 || net->dims[l] % 128) return false;
+    return true;
+}
+}  // namespace
+
+int cr_mlp_forward(const cr_mlp_net* net, int batch, const void* x, int ldx, float* out, int tc, int* err,
+                   void* stream) {
+    if (!mlp_dims_ok(net, batch) || !x || !out) return CR_MLP_EBADSHAPE;
+    const void* in = x;
+    int ld = ldx;
+    for (int l = 0; l < net->layers; ++l) {
+        const bool last = l == net->layers - 1;
+        void* to = last ? (void*)out : net->act[l + 1];
+        const int rc = mlp_gemm_any(last ? CR_MLP_EPI_BIAS_F32 : CR_MLP_EPI_BIAS_RELU_BF16, tc, in, net->w16[l], batch,
+                                    net->dims[l + 1], net->dims[l], ld, net->dims[l], to, net->b[l], nullptr, 0, err,
+                                    stream);
+        if (rc) return rc;
+        in = to;
+        ld = net->dims[l + 1];
+    }
+    return CR_MLP_OK;
+}
+
+int cr_mlp_backward(const cr_mlp_net* net, int batch, const void* x, int ldx, int tc, int* err, void* stream) {
+    if (!mlp_dims_ok(net, batch) || !x || ldx % 8 || !aligned16(x)) return CR_MLP_EBADSHAPE;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int L = net->layers;
+    // gradients down to the first layer's output, through the ReLU whose output was act[l]
+    for (int l = L - 1; l > 0; --l) {
+        const int rc = mlp_gemm_any(CR_MLP_EPI_RELU_MASK_BF16, tc, net->grad[l], net->wt16[l], batch, net->dims[l],
+                                    net->dims[l + 1], net->dims[l + 1], net->dims[l + 1], net->grad[l - 1], nullptr,
+                                    net->act[l], net->dims[l], err, stream);
+        if (rc) return rc;
+    }
+    // dW = grad^T act: both transposed to batch-contiguous rows, and the bias
+    // gradients, kMaxMats / 2 layers to a launch
+    for (int l0 = 0; l0 < L; l0 += kMaxMats / 2) {
+        Mats t{}, c{};
+        for (int l = l0; l < L && l < l0 + kMaxMats / 2; ++l) {
+            const int d_out = net->dims[l + 1], d_in = net->dims[l];
+            auto put = [&](const void* src, int ld, void* dst, int cols) {
+                const int i = t.n++;
+                t.src[i] = (const __nv_bfloat16*)src;
+                t.dst[i] = dst;
+                t.lds[i] = ld;
+                t.ldd[i] = batch;
+                t.rows[i] = batch;
+                t.cols[i] = cols;
+                t.first[i + 1] = t.first[i] + (batch / 64) * (cols / 64);
+            };
+            put(net->grad[l], d_out, net->grad_t[l], d_out);
+            put(l == 0 ? x : net->act[l], l == 0 ? ldx : d_in, net->act_t[l], d_in);
+            const int i = c.n++;
+            c.src[i] = (const __nv_bfloat16*)net->grad[l];
+            c.dst[i] = net->gb[l];
+            c.lds[i] = c.cols[i] = d_out;
+            c.rows[i] = batch;
+            c.first[i + 1] = c.first[i] + d_out / 64;
+        }
+        transpose_mats<<<t.first[t.n], 256, 0, st>>>(t);
+        col_sum_mats<<<c.first[c.n], dim3(32, 32), 0, st>>>(c);
+        if (cudaGetLastError() != cudaSuccess) return CR_MLP_ECUDA;
+    }
+    for (int l = L - 1; l >= 0; --l) {
+        const int rc = mlp_gemm_any(CR_MLP_EPI_F32, tc, net->grad_t[l], net->act_t[l], net->dims[l + 1], net->dims[l],
+                                    batch, batch, batch, net->gw[l], nullptr, nullptr, 0, err, stream);
+        if (rc) return rc;
+    }
+    return CR_MLP_OK;
+}
+
+int cr_mlp_step(const cr_mlp_net* net, float lr, float beta1, float beta2, float eps, int step, float weight_decay,
+                void* stream) {
+    if (!mlp_dims_ok(net, 128) || step < 1) return CR_MLP_EBADSHAPE;
+    for (int l0 = 0; l0 < net->layers; l0 += kMaxMats / 2) {
+        AdamMats t{};
+        for (int l = l0; l < net->layers && l < l0 + kMaxMats / 2; ++l) {
+            const int w = t.n, b = w + 1, d_out = net->dims[l + 1], d_in = net->dims[l];
+            t.n += 2;
+            t.p[w] = net->w[l];
+            t.g[w] = net->gw[l];
+            t.m[w] = net->mw[l];
+            t.v[w] = net->vw[l];
+            t.pb[w] = (__nv_bfloat16*)net->w16[l];
+            t.pt[w] = (__nv_bfloat16*)net->wt16[l];
+            t.rows[w] = d_out;
+            t.cols[w] = d_in;
+            t.first[w + 1] = t.first[w] + (d_out / 64) * (d_in / 64);
+            t.p[b] = net->b[l];
+            t.g[b] = net->gb[l];
+            t.m[b] = net->mb[l];
+            t.v[b] = net->vb[l];
+            t.rows[b] = d_out;
+            t.cols[b] = 1;
+            t.first[b + 1] = t.first[b] + (d_out + 4095) / 4096;
+        }
+        adam_mats<<<t.first[t.n], 256, 0, (cudaStream_t)stream>>>(t, adam_args(lr, beta1, beta2, eps, step),
+                                                                  weight_decay);
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
+}
+
+int cr_mlp_ensemble_stats(const float* const* preds, int members, long long n, float scale, float mid, float lo,
+                          float hi, float* mean, float* spread, void* stream) {
+    if (!preds || members < 1 || members > kMaxMembers || n <= 0 || n % 4 || !aligned16(mean) || !aligned16(spread))
+        return CR_MLP_EBADSHAPE;
+    Members p{};
+    for (int k = 0; k < members; ++k) {
+        if (!preds[k] || !aligned16(preds[k])) return CR_MLP_EBADSHAPE;
+        p.out[k] = preds[k];
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    const long long n4 = n / 4, want = (n4 + 255) / 256;
+    const int grid = (int)(want < 148 * 16 ? want : 148 * 16);
+    auto m4 = (float4*)mean;
+    auto s4 = (float4*)spread;
+    switch (members) {
+        case 2: ensemble_stats<2><<<grid, 256, 0, st>>>(p, members, n4, scale, mid, lo, hi, m4, s4); break;
+        case 3: ensemble_stats<3><<<grid, 256, 0, st>>>(p, members, n4, scale, mid, lo, hi, m4, s4); break;
+        case 4: ensemble_stats<4><<<grid, 256, 0, st>>>(p, members, n4, scale, mid, lo, hi, m4, s4); break;
+        default: ensemble_stats<0><<<grid, 256, 0, st>>>(p, members, n4, scale, mid, lo, hi, m4, s4); break;
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
 }
 

@@ -79,6 +79,26 @@ _SIGS = {
                        ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
                        ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p],
 }
+
+
+class _Net(ctypes.Structure):
+    """cr_mlp_net: host arrays of device pointers, one per layer."""
+    _fields_ = [("layers", ctypes.c_int), ("dims", ctypes.c_void_p)] + [
+        (k, ctypes.c_void_p) for k in ("w", "b", "w16", "wt16", "gw", "gb", "mw", "vw", "mb", "vb", "act", "grad",
+                                       "act_t", "grad_t")]
+
+
+_SIGS.update({
+    "cr_mlp_forward": [ctypes.POINTER(_Net), ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p,
+                       ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p],
+    "cr_mlp_backward": [ctypes.POINTER(_Net), ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_int,
+                        ctypes.c_void_p, ctypes.c_void_p],
+    "cr_mlp_step": [ctypes.POINTER(_Net), ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                    ctypes.c_int, ctypes.c_float, ctypes.c_void_p],
+    "cr_mlp_ensemble_stats": [ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_float,
+                              ctypes.c_float, ctypes.c_float, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p],
+})
+MAX_MEMBERS = 64  # of cr_mlp_ensemble_stats
 # Contractions with N a multiple of 256 and K of 64 run on the tcgen05 tensor
 # cores (cr_mlp_gemm_tc); the others on the mma.sync kernel (cr_mlp_gemm).
 USE_TCGEN05 = True
@@ -195,54 +215,50 @@ class MLP:
             H = [None] + [torch.empty(B, d, dtype=torch.bfloat16, device=dev) for d in self.dims[1:-1]]
             out = torch.empty(B, self.dims[-1], dtype=torch.float32, device=dev)
             dH = [torch.empty(B, d, dtype=torch.bfloat16, device=dev) for d in self.dims[1:]]
-            T = torch.empty(max(self.dims) * B, dtype=torch.bfloat16, device=dev)
-            T2 = torch.empty(max(self.dims) * B, dtype=torch.bfloat16, device=dev)
+            T = [torch.empty(d, B, dtype=torch.bfloat16, device=dev) for d in self.dims[1:]]
+            T2 = [torch.empty(d, B, dtype=torch.bfloat16, device=dev) for d in self.dims[:-1]]
             self._bufs[B] = (H, out, dH, T, T2)
         return self._bufs[B]
+
+    def _net(self, B=None, **tensors):
+        """cr_mlp_net of the tensors as they are now (and of the batch's buffers)."""
+        if B is not None:
+            H, _, dH, T, T2 = self._buffers(B)
+            tensors.update(act=H, grad=dH, act_t=T2, grad_t=T)
+        net = _Net(layers=len(self.W))
+        keep = [(ctypes.c_int * len(self.dims))(*self.dims)]
+        net.dims = ctypes.addressof(keep[0])
+        for name, lst in tensors.items():
+            keep.append((ctypes.c_void_p * len(lst))(*[t.data_ptr() if t is not None else None for t in lst]))
+            setattr(net, name, ctypes.addressof(keep[-1]))
+        net.keep = keep
+        return net
 
     def forward(self, X):
         """X: [B, d_in] bf16 (B a multiple of 128) -> output [B, d_out] f32 (a reused buffer)."""
         B = X.shape[0]
         H, out, _, _, _ = self._buffers(B)
+        assert X.shape[1] == self.dims[0]
         H[0] = X
-        L = len(self.W)
-        for l in range(L):
-            if l < L - 1:
-                gemm(EPI_BIAS_RELU_BF16, H[l], self.Wb[l], H[l + 1], bias=self.b[l])
-            else:
-                gemm(EPI_BIAS_F32, H[l], self.Wb[l], out, bias=self.b[l])
+        _ok(kernels().cr_mlp_forward(self._net(B, w16=self.Wb, b=self.b), B, _p(X), X.stride(0), _p(out),
+                                     int(USE_TCGEN05), _p(tc_error_flag()), _stream()), "cr_mlp_forward")
         return out
 
     def backward(self, dout):
         """dout: [B, d_out] bf16 gradient of the loss at the output; fills gW, gb."""
         B = dout.shape[0]
-        H, _, dH, T, T2 = self._buffers(B)
-        L = len(self.W)
-        if dH[L - 1].data_ptr() != dout.data_ptr():
-            dH[L - 1].copy_(dout)
-        for l in range(L - 1, -1, -1):
-            d_out, d_in = self.dims[l + 1], self.dims[l]
-            g = dH[l]
-            # dW = g^T X: both transposed to K(=batch)-contiguous rows
-            gT = T[: d_out * B].view(d_out, B)
-            xT = T2[: d_in * B].view(d_in, B)
-            transpose(g, gT)
-            transpose(H[l], xT)
-            gemm(EPI_F32, gT, xT, self.gW[l])
-            _ok(kernels().cr_mlp_col_sum(_p(g), g.stride(0), B, d_out, _p(self.gb[l]), _stream()), "cr_mlp_col_sum")
-            if l > 0:
-                # dX = g W through the ReLU whose output was H[l]
-                gemm(EPI_RELU_MASK_BF16, g, self.WTb[l], dH[l - 1], mask=H[l])
+        H, _, dH, _, _ = self._buffers(B)
+        if dH[-1].data_ptr() != dout.data_ptr():
+            dH[-1].copy_(dout)
+        X = H[0]
+        _ok(kernels().cr_mlp_backward(self._net(B, wt16=self.WTb, gw=self.gW, gb=self.gb), B, _p(X), X.stride(0),
+                                      int(USE_TCGEN05), _p(tc_error_flag()), _stream()), "cr_mlp_backward")
 
     def step(self, lr, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
         self.t += 1
-        k = kernels()
-        for l in range(len(self.W)):
-            _ok(k.cr_mlp_adam(_p(self.W[l]), _p(self.gW[l]), _p(self.mW[l]), _p(self.vW[l]), _p(self.Wb[l]),
-                              self.W[l].numel(), lr, beta1, beta2, eps, self.t, weight_decay, _stream()), "adam")
-            _ok(k.cr_mlp_adam(_p(self.b[l]), _p(self.gb[l]), _p(self.mb[l]), _p(self.vb[l]), None,
-                              self.b[l].numel(), lr, beta1, beta2, eps, self.t, 0.0, _stream()), "adam")
-            transpose(self.Wb[l], self.WTb[l])
+        net = self._net(w=self.W, b=self.b, w16=self.Wb, wt16=self.WTb, gw=self.gW, gb=self.gb, mw=self.mW,
+                        vw=self.vW, mb=self.mb, vb=self.vb)
+        _ok(kernels().cr_mlp_step(net, lr, beta1, beta2, eps, self.t, weight_decay, _stream()), "cr_mlp_step")
 
     def grad_buffer(self, B):
         """The bf16 buffer backward() reads the output gradient from."""
@@ -449,10 +465,17 @@ class Ensemble:
         spread = torch.empty(n, NZ_OUT * NR_OUT, device=X.device)
         for s in range(0, n, chunk):
             xb = X[s: s + chunk]
-            preds = torch.stack([m.forward(xb).clone() for m in self.models]) * TL_SCALE + TL_MID
-            preds.clamp_(TL_LO, TL_HI)
-            mean[s: s + chunk] = preds.mean(0)
-            spread[s: s + chunk] = preds.std(0, unbiased=False)
+            # every member's output stays in its own buffer until the statistics have read it
+            preds = [m.forward(xb) for m in self.models]
+            if len(preds) <= MAX_MEMBERS:
+                ptrs = (ctypes.c_void_p * len(preds))(*[p.data_ptr() for p in preds])
+                _ok(kernels().cr_mlp_ensemble_stats(ptrs, len(preds), preds[0].numel(), TL_SCALE, TL_MID, TL_LO, TL_HI,
+                                                    _p(mean[s: s + chunk]), _p(spread[s: s + chunk]), _stream()),
+                    "cr_mlp_ensemble_stats")
+                continue
+            tl = (torch.stack(preds) * TL_SCALE + TL_MID).clamp_(TL_LO, TL_HI)
+            mean[s: s + chunk] = tl.mean(0)
+            spread[s: s + chunk] = tl.std(0, unbiased=False)
         if check:
             check_tc_flag()
         return mean.view(n, NZ_OUT, NR_OUT), spread.view(n, NZ_OUT, NR_OUT)

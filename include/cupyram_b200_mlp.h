@@ -67,6 +67,49 @@ int cr_mlp_mse_grad(const float* pred, const void* target, const unsigned char* 
 int cr_mlp_adam(float* p, const float* g, float* m, float* v, void* p_bf16, long long n, float lr, float beta1,
                 float beta2, float eps, int step, float weight_decay, void* stream);
 
+/* A fully connected ReLU network of `layers` layers, dims[0] inputs to
+ * dims[layers] outputs (all multiples of 128), as the three calls below take
+ * it: host arrays of device pointers, one per layer l, matrices row-major and
+ * dense.  Arrays that a call does not use may be NULL. */
+typedef struct cr_mlp_net {
+    int layers;
+    const int* dims;      /* [layers + 1]                                       */
+    float* const* w;      /* f32 weights [dims[l+1]][dims[l]]                   */
+    float* const* b;      /* f32 biases                                         */
+    void* const* w16;     /* bf16 copy of w                                     */
+    void* const* wt16;    /* its transpose [dims[l]][dims[l+1]]                 */
+    float* const* gw;     /* gradients                                          */
+    float* const* gb;
+    float* const* mw;     /* Adam's moments                                     */
+    float* const* vw;
+    float* const* mb;
+    float* const* vb;
+    void* const* act;     /* bf16 [batch][dims[l]]: input of layer l, l >= 1    */
+    void* const* grad;    /* bf16 [batch][dims[l+1]]: gradient at its output    */
+    void* const* act_t;   /* bf16 [dims[l]][batch] (scratch)                    */
+    void* const* grad_t;  /* bf16 [dims[l+1]][batch] (scratch)                  */
+} cr_mlp_net;
+
+/* out (f32) = the network's outputs for x (bf16, row stride ldx); fills act.
+ * tc: contractions with N a multiple of 256 and K of 64 on the tcgen05 kernel. */
+int cr_mlp_forward(const cr_mlp_net* net, int batch, const void* x, int ldx, float* out, int tc, int* err,
+                   void* stream);
+
+/* From grad[layers-1] (set by the caller) and act: every grad, gw and gb. */
+int cr_mlp_backward(const cr_mlp_net* net, int batch, const void* x, int ldx, int tc, int* err, void* stream);
+
+/* One Adam step of every layer (cr_mlp_adam; weight_decay on the weights
+ * only), with the bf16 copies and their transposes. */
+int cr_mlp_step(const cr_mlp_net* net, float lr, float beta1, float beta2, float eps, int step, float weight_decay,
+                void* stream);
+
+/* mean[i] and spread[i] (standard deviation, divided by members) over the
+ * members (at most 64) of t = clamp(preds[k][i] * scale + mid, lo, hi), for n
+ * values (a multiple of 4, 16-byte aligned arrays).  preds: host array of
+ * device pointers. */
+int cr_mlp_ensemble_stats(const float* const* preds, int members, long long n, float scale, float mid, float lo,
+                          float hi, float* mean, float* spread, void* stream);
+
 /* dst = BF16(src) for n values. */
 int cr_mlp_to_bf16(const float* src, void* dst, long long n, void* stream);
 
