@@ -82,8 +82,11 @@ struct RegCtl {
     long long col;           // the ray's column
     double cfact, a1, a2;
     int seg;                 // rows of a segment of the factorisation
+    int env, n_bt, n_rss, n_rsb;
+    double dr, dz;
+    const double *rb, *zb, *rp_ss, *rp_sb;
 };
-constexpr unsigned kCtlBytes = 192;
+constexpr unsigned kCtlBytes = 256;
 static_assert(sizeof(RegCtl) <= kCtlBytes, "RegCtl must fit its slot");
 
 // Shared memory of a CTA (offsets in bytes; every CTA of a cluster uses the
@@ -301,36 +304,68 @@ __device__ __noinline__ double2 reg_recurrence(const double2* D, int P, double2 
     return c2(-wp.x, -wp.y);
 }
 
+// Affine scan over the lanes, h_l += M_l h_{l -/+ d}: the multipliers of level
+// i are at tab + 512 i, those of the last level (sx) only hold in one half of
+// the warp.  Each level's multiplier is read a level ahead of its use.
+template <bool UP>
+__device__ __forceinline__ double2 lane_scan(double2 h, unsigned tab, double2 m, double2 sx, int l) {
+#pragma unroll
+    for (int lev = 0; lev < 4; ++lev) {
+        const double2 next = lev < 3 ? lds2(tab + (lev + 1) * 512u) : c2(0.0, 0.0);
+        h = vfma(m, UP ? shfl2_down(h, 1 << lev) : shfl2_up(h, 1 << lev), h);
+        m = next;
+    }
+    const double2 t = UP ? shfl2_down(h, 16) : shfl2_up(h, 16);
+    const bool in = UP ? l < 16 : l >= 16;
+    return vfma(in ? sx : c2(0.0, 0.0), t, h);
+}
+
 // Weights of the slices' h and y in this slice's gin and xin, from every
 // slice's (A, Z, V): gin(c) = sum_{i<c} [A over i+1..c-1] h_i and
 // xin(c) = sum_{j>c} [Z over c+1..j-1] (y_j + V_j gin(j)).
 __device__ __noinline__ void reg_weights(double2* tot, double2* WA, double2* WB, int C, int c) {
     cg::cluster_group cl = cg::this_cluster();
     const int i = threadIdx.x & 31;
-    double2 A = c2(1.0, 0.0), Z = A, V = c2(0.0, 0.0);
+    const double2 one = c2(1.0, 0.0), zero = c2(0.0, 0.0);
+    double2 A = one, Z = one, V = zero;
     if (i < C) {
         const double2* f = cl.map_shared_rank(tot, i);
         A = f[0];
         Z = f[1];
         V = f[2];
     }
-    double2 g = c2(0.0, 0.0), x = g, y = g, pf = c2(1.0, 0.0), pb = pf;
-#pragma unroll 1
-    for (int j = 0; j < C; ++j) {
-        const double2 Aj = shfl2(A, j), Zj = shfl2(Z, j), Vj = shfl2(V, j);
-        if (j == c && i < c) g = pf;
-        if (j > c) {
-            if (i == j) y = pb;
-            if (i < j) x = vfma(cmul(pb, Vj), pf, x);
-            pb = cmul(pb, Zj);
+    // lane i: the products of A over i .. c - 1 and of Z over c + 1 .. i, and then
+    // without the first and the last
+    double2 pa = i < c ? A : one, pz = i > c ? Z : one;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        const double2 qa = shfl2(pa, min(i + d, 31)), qz = shfl2(pz, max(i - d, 0));
+        pa = i + d < 32 ? cmul(pa, qa) : pa;
+        pz = i >= d ? cmul(pz, qz) : pz;
+    }
+    const double2 g = shfl2(pa, min(i + 1, 31)), y = shfl2(pz, max(i - 1, 0));
+    // h of slice i reaches xin through V of every slice below both i and this one:
+    // x_i = t_{i+1} + A_{i+1} x_{i+1}, t_j = [Z over c+1..j-1] V_j; scanned upwards
+    // as maps x -> M x + T, each lane's own map that of lane i + 1
+    double2 t = i > c && i < C ? cmul(y, V) : zero;
+    double2 T = shfl2_down(t, 1), M = shfl2_down(A, 1);
+    if (i + 1 >= C) {
+        T = zero;
+        M = one;
+    }
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        const double2 qm = shfl2(M, min(i + d, 31)), qt = shfl2(T, min(i + d, 31));
+        if (i + d < 32) {
+            T = vfma(M, qt, T);
+            M = cmul(M, qm);
         }
-        if (i < j) pf = cmul(pf, Aj);
     }
     if (i < 16) {
-        WA[i] = g;
-        WA[16 + i] = x;
-        WB[i] = c2(0.0, 0.0);
-        WB[16 + i] = y;
+        WA[i] = i < c ? g : zero;
+        WA[16 + i] = i < C ? T : zero;
+        WB[i] = zero;
+        WB[16 + i] = i > c && i < C ? y : zero;
     }
 }
 
@@ -400,7 +435,7 @@ __device__ __forceinline__ void reg_factor(const ColArgs& a, const RegCtx& x, cg
         }
         x.own(O::V)[l] = v;
         // A and Z over 1, 2, .. lanes, and over all lanes above (EA) or below (EZ)
-#pragma unroll 1
+#pragma unroll
         for (int lev = 0; lev < 5; ++lev) {
             const int d = 1 << lev;
             if (lev < 4) {
@@ -421,10 +456,9 @@ __device__ __forceinline__ void reg_factor(const ColArgs& a, const RegCtx& x, cg
         // EV: v of the lane per unit of gin
         v = cmul(v, ea);
         __syncwarp();
-#pragma unroll 1
-        for (int lev = 0; lev < 5; ++lev) {
-            const double2 m = lev < 4 ? x.own(O::SU)[lev * 32 + l] : (l < 16 ? x.own(O::SX)[l] : c2(0.0, 0.0));
-            v = vfma(m, shfl2_down(v, 1 << lev), v);
+        {
+            const unsigned tl = x.tm32 + 16u * (unsigned)l;
+            v = lane_scan<true>(v, tl + O::SU, lds2(tl + O::SU), lds2(tl + O::SX), l);
         }
         const double2 ev = shfl2_down(v, 1);
         x.own(O::EV)[l] = l == 31 ? c2(0.0, 0.0) : ev;
@@ -442,13 +476,18 @@ __device__ __forceinline__ void reg_factor(const ColArgs& a, const RegCtx& x, cg
     __syncthreads();
 }
 
-// Initial profiles or the rows [lo, hi] again, split over the cluster.
-__device__ __noinline__ void reg_assemble(const ColArgs& a, int rid, int C, int c, int ss, int sb, int iz, int lo,
-                                          int hi) {
-    const RayDev ry = a.rays[rid];
-    const EnvPtrs e = env_ptrs(a.envs[ry.env], a.pool);
-    for (int i = lo + c + C * (int)threadIdx.x; i <= hi; i += C * blockDim.x)
-        assemble_rows(ry, e, ss, sb, iz, i, i, a.f1, a.f2, a.f3, a.ksq);
+// The rows of [lo, hi] that the CTA reads - its slice and one row each side -
+// assembled by its own threads.  A row between two slices is written by both
+// CTAs, with the same values, and each reads what it wrote: no CTA waits.
+__device__ __noinline__ void reg_assemble(const ColArgs& a, const RegCtl* ctl, int lo, int hi) {
+    const int first = max(lo, ctl->R0 - 1), last = min(hi, ctl->R1 + 1);
+    if (first + (int)threadIdx.x <= last) {
+        const RayDev ry = a.rays[ctl->rid];
+        const EnvPtrs e = env_ptrs(a.envs[ctl->env], a.pool);
+        for (int i = first + (int)threadIdx.x; i <= last; i += blockDim.x)
+            assemble_rows(ry, e, ctl->ss, ctl->sb, ctl->iz, i, i, a.f1, a.f2, a.f3, a.ksq);
+    }
+    __syncthreads();
 }
 
 // The self-starter's delta in the slice and its halo (cupyram.py:1008-1022).
@@ -484,23 +523,22 @@ __device__ __noinline__ void reg_source(const ColArgs& a, RegCtx x) {
 // the operator: the next profile, bottom segment or stability range lies
 // further on, and the bottom's depth index (linear in range within a segment)
 // stays in its cell; both bounds keep a step's margin for rounding.
-__device__ __noinline__ void reg_updat(const ColArgs& a, int rn, RegCtl* ctl) {
-    const RayDev& ry = a.rays[ctl->rid];
-    const EnvPtrs e = env_ptrs(a.envs[ry.env], a.pool);
-    const double r = (double)(rn + 1) * ry.dr;
+__device__ __noinline__ void reg_updat(int rn, RegCtl* ctl) {
+    const RegCtl& e = *ctl;
+    const double dr = e.dr, r = (double)(rn + 1) * dr;
     bool reprofile = false;
     int iz = ctl->iz, ss = ctl->ss, sb = ctl->sb, bt = ctl->bt, set = ctl->set == 1 ? 2 : ctl->set;
     double stay = 1e9;  // steps that cannot change anything
-    auto event = [&](double v) { stay = fmin(stay, floor(v / ry.dr) - 2.0 - (double)rn); };
+    auto event = [&](double v) { stay = fmin(stay, floor(v / dr) - 2.0 - (double)rn); };
     if (e.n_bt > 1) {
         while (bt < e.n_bt - 1 && r >= e.rb[bt + 1]) ++bt;
         const int b1 = min(bt + 1, e.n_bt - 1);
         const double r0 = e.rb[bt], r1 = e.rb[b1], z0 = e.zb[bt], z1 = e.zb[b1];
-        const double zc = (b1 == bt) ? z0 : z0 + (r + 0.5 * ry.dr - r0) * (z1 - z0) / (r1 - r0);
-        iz = max(1, min(ry.nz - 1, (int)floor(zc / ry.dz)));
+        const double zc = (b1 == bt) ? z0 : z0 + (r + 0.5 * dr - r0) * (z1 - z0) / (r1 - r0);
+        iz = max(1, min(e.nz - 1, (int)floor(zc / e.dz)));
         if (b1 != bt) {
             event(r1);
-            const double f = zc / ry.dz, per = (z1 - z0) / (r1 - r0) * ry.dr / ry.dz;
+            const double f = zc / e.dz, per = (z1 - z0) / (r1 - r0) * dr / e.dz;
             if (per > 0.0) stay = fmin(stay, floor((floor(f) + 1.0 - f) / per) - 1.0);
             if (per < 0.0) stay = fmin(stay, floor((floor(f) - f) / per) - 1.0);
         }
@@ -524,7 +562,7 @@ __device__ __noinline__ void reg_updat(const ColArgs& a, int rn, RegCtl* ctl) {
     }
     if (rs < 1e300) event(rs);
     ctl->lo = reprofile ? 0 : min(ctl->iz, iz) + 1;
-    ctl->hi = reprofile ? ry.nz + 1 : max(ctl->iz, iz);  // iz unchanged: lo > hi
+    ctl->hi = reprofile ? e.nz + 1 : max(ctl->iz, iz);  // iz unchanged: lo > hi
     ctl->refactor = reprofile || iz != ctl->iz || set != ctl->set;
     ctl->iz = iz;
     ctl->ss = ss;
@@ -578,22 +616,6 @@ __device__ __noinline__ void reg_outputs(const ColArgs& a, RegCtl* ctl) {
     ctl->ndz = (unsigned)ry.ndz;
     ctl->ndz_inv = ry.ndz > 1 ? (unsigned)((0x100000000ull + ry.ndz - 1) / (unsigned)ry.ndz) : 0u;
     ctl->nvz = ry.nvz;
-}
-
-// Affine scan over the lanes, h_l += M_l h_{l -/+ d}: the multipliers of level
-// i are at tab + 512 i, those of the last level (sx) only hold in one half of
-// the warp.  Each level's multiplier is read a level ahead of its use.
-template <bool UP>
-__device__ __forceinline__ double2 lane_scan(double2 h, unsigned tab, double2 m, double2 sx, int l) {
-#pragma unroll
-    for (int lev = 0; lev < 4; ++lev) {
-        const double2 next = lev < 3 ? lds2(tab + (lev + 1) * 512u) : c2(0.0, 0.0);
-        h = vfma(m, UP ? shfl2_down(h, 1 << lev) : shfl2_up(h, 1 << lev), h);
-        m = next;
-    }
-    const double2 t = UP ? shfl2_down(h, 16) : shfl2_up(h, 16);
-    const bool in = UP ? l < 16 : l >= 16;
-    return vfma(in ? sx : c2(0.0, 0.0), t, h);
 }
 
 // The sum over N pairs of terms of the rows j = k, k + terms, .. of this lane
@@ -860,6 +882,16 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
         ctl->next = 0;
         ctl->dead = 0;
         ctl->rs = ry.rs;
+        ctl->env = ry.env;
+        ctl->dr = ry.dr;
+        ctl->dz = ry.dz;
+        ctl->n_bt = e.n_bt;
+        ctl->n_rss = e.n_rss;
+        ctl->n_rsb = e.n_rsb;
+        ctl->rb = e.rb;
+        ctl->zb = e.zb;
+        ctl->rp_ss = e.rp_ss;
+        ctl->rp_sb = e.rp_sb;
         misc[1] = misc[2] = misc[3] = c2(0.0, 0.0);
         for (int k = 0; k < 2 * (int)(blockDim.x >> 5); ++k)
             mbar_init1(x.at<unsigned long long>(O::term0 + (unsigned)(k >> 1) * O::term + O::bar) + (k & 1));
@@ -868,13 +900,12 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
     for (int p = threadIdx.x; p < 32 * L; p += blockDim.x) x.at<double2>(O::U)[p] = c2(0.0, 0.0);
     x.own(O::mail)[x.lane] = x.own(O::mail)[32 + x.lane] = c2(0.0, 0.0);
     __syncthreads();
-    reg_assemble(a, ctl->rid, x.C, x.c, 0, 0, ctl->iz, 0, ctl->nz + 1);
+    reg_assemble(a, ctl, 0, ctl->nz + 1);
     if (threadIdx.x == 0) {
         reg_source<L>(a, x);
         reg_outputs<L>(a, ctl);
     }
-    __threadfence();
-    cl.sync();
+    cl.sync();  // every CTA's mailboxes are ready
     reg_load_f3<L>(a, x, 0, ctl->nz + 1);
     const int n = ctl->n;
     {
@@ -909,15 +940,13 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
         stop = s == 0 ? 2 : 3;
         if (s >= 3) {
             __syncthreads();
-            if (threadIdx.x == 0) reg_updat(a, s - 3, ctl);
+            if (threadIdx.x == 0) reg_updat(s - 3, ctl);
             __syncthreads();
             stop = min(steps, ctl->next + 3);
             want = ctl->set;
             refactor = ctl->refactor;
             if (ctl->lo <= ctl->hi) {
-                reg_assemble(a, ctl->rid, x.C, x.c, ctl->ss, ctl->sb, ctl->iz, ctl->lo, ctl->hi);
-                __threadfence();
-                cl.sync();
+                reg_assemble(a, ctl, ctl->lo, ctl->hi);
                 reg_load_f3<L>(a, x, ctl->lo, ctl->hi);
             }
         }
