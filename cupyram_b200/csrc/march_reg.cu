@@ -99,7 +99,8 @@ struct RegOff {
     static constexpr unsigned ck = 0;                      // residues of the active set
     static constexpr unsigned misc = ck + 16 * CR_MAX_NP;  // c_inf, u of row R0 - 1, u of row R1 + 1, zero
     static constexpr unsigned ctl = misc + 64;
-    static constexpr unsigned U = ctl + kCtlBytes;         // field of the slice, slot [j][lane]
+    static constexpr unsigned edges = ctl + kCtlBytes;     // [32] offsets of the field above (low half) and below
+    static constexpr unsigned U = edges + 128;             // field of the slice, slot [j][lane]
     static constexpr unsigned term0 = U + 16 * P;
     // of a term's region
     static constexpr unsigned Q = 0;                       // [P] a1 / den
@@ -167,6 +168,11 @@ __device__ __forceinline__ bool mail_wait(unsigned bar, unsigned bytes, unsigned
 __device__ __forceinline__ double2 lds2(unsigned addr) {
     double2 v;
     asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned lds1(unsigned addr) {
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
     return v;
 }
 __device__ __forceinline__ void sts2(unsigned addr, double2 v) {
@@ -305,16 +311,20 @@ __device__ __noinline__ double2 reg_recurrence(const double2* D, int P, double2 
 }
 
 // Affine scan over the lanes, h_l += M_l h_{l -/+ d}: the multipliers of level
-// i are at tab + 512 i, those of the last level (sx) only hold in one half of
-// the warp.  Each level's multiplier is read a level ahead of its use.
-template <bool UP>
-__device__ __forceinline__ double2 lane_scan(double2 h, unsigned tab, double2 m, double2 sx, int l) {
+// i are at tab + 512 i, those of the last level (at last) only hold in one half
+// of the warp.  AHEAD: each level's multiplier is read a level before its use,
+// the first (m) and the last (sx) by the caller.
+template <bool UP, bool AHEAD>
+__device__ __forceinline__ double2 lane_scan(double2 h, unsigned tab, unsigned last, double2 m, double2 sx, int l) {
 #pragma unroll
     for (int lev = 0; lev < 4; ++lev) {
-        const double2 next = lev < 3 ? lds2(tab + (lev + 1) * 512u) : c2(0.0, 0.0);
+        double2 next = c2(0.0, 0.0);
+        if (AHEAD && lev < 3) next = lds2(tab + (lev + 1) * 512u);
+        if (!AHEAD) m = lds2(tab + lev * 512u);
         h = vfma(m, UP ? shfl2_down(h, 1 << lev) : shfl2_up(h, 1 << lev), h);
         m = next;
     }
+    if (!AHEAD) sx = lds2(last);
     const double2 t = UP ? shfl2_down(h, 16) : shfl2_up(h, 16);
     const bool in = UP ? l < 16 : l >= 16;
     return vfma(in ? sx : c2(0.0, 0.0), t, h);
@@ -458,7 +468,7 @@ __device__ __forceinline__ void reg_factor(const ColArgs& a, const RegCtx& x, cg
         __syncwarp();
         {
             const unsigned tl = x.tm32 + 16u * (unsigned)l;
-            v = lane_scan<true>(v, tl + O::SU, lds2(tl + O::SU), lds2(tl + O::SX), l);
+            v = lane_scan<true, true>(v, tl + O::SU, 0u, lds2(tl + O::SU), lds2(tl + O::SX), l);
         }
         const double2 ev = shfl2_down(v, 1);
         x.own(O::EV)[l] = l == 31 ? c2(0.0, 0.0) : ev;
@@ -653,11 +663,10 @@ __device__ __forceinline__ void reg_sum(const ColArgs& a, const RegCtx& x, doubl
 
 // One range step of the active set; out >= 0: the step's field is output
 // `out` (outpt.py:11-57; transmission loss follows at the end, reg_tl).
-// edges: offsets of the field above the lane's rows (low half) and below.
+// step: index of the step, the self-starter's three included.
 template <int L>
 __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int na, const double2 (&al)[L],
-                                         const double2 (&mw)[L], unsigned edges, unsigned raddr, unsigned& count,
-                                         int out) {
+                                         const double2 (&mw)[L], int step, int out) {
     using O = RegOff<L>;
     constexpr unsigned P16 = 512u * L;  // bytes of a per-row table
     const int k = x.term, l = x.lane, terms = (int)(blockDim.x >> 5);
@@ -666,63 +675,91 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
     const int half = (na + 1) >> 1;
     if (k < na) {
         const unsigned tl = tm + 16u * (unsigned)l;  // this lane's entries of the term's tables
+        // Tables are read ahead of their use where registers are left for it; with 12
+        // rows a lane the factors and the workspace take 144 of the 168.
+        constexpr bool kAhead = L <= 10;
+        const int npad = x.npad;
         double2 g[L];
         // h down the lane's rows, then y up
-        double2 h = c2(0.0, 0.0), y = h, m;
+        double2 h = c2(0.0, 0.0), y = h, m, sx;
         {
+            const unsigned edges = lds1(sm + O::edges + 4u * (unsigned)l);
             double2 up = lds2(sm + (edges & 0xffffu));
 #pragma unroll
             for (int j = 0; j < L; ++j) g[j] = lds2(us + j * 512u);
-            const double2 after = lds2(sm + (edges >> 16));
-            double2 q0 = lds2(tl + O::Q), q1 = L > 1 ? lds2(tl + O::Q + 512u) : q0;
+            double2 after, q0, q1;
+            if (kAhead) {
+                after = lds2(sm + (edges >> 16));
+                q0 = lds2(tl + O::Q);
+                if (L > 1) q1 = lds2(tl + O::Q + 512u);
+            }
 #pragma unroll
             for (int j = 0; j < kMaxPad && j < L; ++j)
-                if (j < x.npad) g[j] = up;
+                if (j < npad) g[j] = up;
 #pragma unroll
             for (int j = 0; j < L; ++j) {
-                const double2 uc = g[j], un = j + 1 < L ? g[j + 1 < L ? j + 1 : 0] : after, q = q0;
-                q0 = q1;
-                if (j + 2 < L) q1 = lds2(tl + O::Q + (j + 2) * 512u);
+                double2 q;
+                if (kAhead) {
+                    q = q0;
+                    q0 = q1;
+                    if (j + 2 < L) q1 = lds2(tl + O::Q + (j + 2) * 512u);
+                } else {
+                    q = lds2(tl + O::Q + j * 512u);
+                    if (j + 1 == L) after = lds2(sm + (edges >> 16));
+                }
+                const double2 uc = g[j], un = j + 1 < L ? g[j + 1 < L ? j + 1 : 0] : after;
                 const double2 b = c2(fma(4.0, uc.x, up.x + un.x), fma(4.0, uc.y, up.y + un.y));
                 h = vfma(al[j], h, cmul(q, b));
                 up = uc;
                 g[j] = h;
             }
-            m = lds2(tl + O::SD);
+            if (kAhead) m = lds2(tl + O::SD);
 #pragma unroll
             for (int j = L - 1; j >= 0; --j)
-                y = vfma(mw[j], y, (j < kMaxPad && j < x.npad) ? c2(0.0, 0.0) : g[j]);
+                y = vfma(mw[j], y, (j < kMaxPad && j < npad) ? c2(0.0, 0.0) : g[j]);
         }
         // e of every lane, the slice alone
-        const double2 sx = lds2(tl + O::SX);
-        h = lane_scan<false>(h, tl + O::SD, m, sx, l);
-        const double2 V = lds2(tl + O::V);
-        m = lds2(tl + O::SU);
+        if (kAhead) sx = lds2(tl + O::SX);
+        h = lane_scan<false, kAhead>(h, tl + O::SD, tl + O::SX, m, sx, l);
         double2 e = shfl2_up(h, 1);
         if (l == 0) e = c2(0.0, 0.0);
-        const unsigned box = count & 1u, par = (count >> 1) & 1u;
-        ++count;
-        const unsigned to = raddr + 512u * box;
-        const unsigned to_bar = raddr - 32u * (unsigned)x.c + (O::bar - O::mail) + 8u * box;
+        // the mailbox of this step: the two alternate over the term's active steps
+        const unsigned count = (unsigned)(k == 0 ? step : step - 2), box = count & 1u, par = (count >> 1) & 1u;
+        const unsigned to = x.C > 1 ? remote_addr(tm + O::mail + 512u * box + 32u * (unsigned)x.c,
+                                                  (unsigned)min(l, x.C - 1)) : 0u;
+        const unsigned to_bar = to - 512u * box - 32u * (unsigned)x.c + (O::bar - O::mail) + 8u * box;
         if (x.C > 1) {
             const double2 t = shfl2(h, 31);
             if (l < x.C) mail_send(to, to_bar, t);
         }
         // v of every lane, the slice alone
-        y = lane_scan<true>(vfma(V, e, y), tl + O::SU, m, sx, l);
+        const double2 V = lds2(tl + O::V);
+        if (kAhead) m = lds2(tl + O::SU);
+        y = lane_scan<true, kAhead>(vfma(V, e, y), tl + O::SU, tl + O::SX, m, sx, l);
         double2 v = shfl2_down(y, 1);
         if (l == 31) v = c2(0.0, 0.0);
-        double2 gin = c2(0.0, 0.0), xin = gin;
         if (x.C > 1) {
             const double2 t = shfl2(y, 0);
             if (l < x.C) mail_send(to + 16u, to_bar, t);
-            const double2 wa = lds2(tl + O::WA), wb = lds2(tl + O::WB);
+            double2 wa, wb, ea, ez, ev;
+            if (kAhead) {
+                wa = lds2(tl + O::WA);
+                wb = lds2(tl + O::WB);
+            }
             if (!ctl->dead && !mail_wait(tm + O::bar + 8u * box, 32u * (unsigned)x.C, par, l)) ctl->dead = 1;
             // lanes 0..15 fold gin, lanes 16..31 xin: lane j the values of CTA j % 16
             // (the weights of CTAs that are not there, and of y in gin, are zero)
             const unsigned mb = tm + O::mail + 512u * box + 32u * (unsigned)(l & 15);
+            if (!kAhead) {
+                wa = lds2(tl + O::WA);
+                wb = lds2(tl + O::WB);
+            }
             const double2 mh = lds2(mb), my = lds2(mb + 16u);
-            const double2 ea = lds2(tl + O::EA), ez = lds2(tl + O::EZ), ev = lds2(tl + O::EV);
+            if (kAhead) {
+                ea = lds2(tl + O::EA);
+                ez = lds2(tl + O::EZ);
+                ev = lds2(tl + O::EV);
+            }
             double2 f = vfma(wb, my, cmul(wa, mh));
             if (x.C > 4) {
                 f = cadd(f, shfl2_xor(f, 8));
@@ -730,10 +767,16 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
             }
             f = cadd(f, shfl2_xor(f, 2));
             f = cadd(f, shfl2_xor(f, 1));
-            gin = shfl2(f, 0);
-            xin = shfl2(f, 16);
+            const double2 gin = shfl2(f, 0), xin = shfl2(f, 16);
+            // for the halo rows, once the lane's x are known
+            if (l == 0) sts2(tm + O::xh, gin);
+            if (l == 0) sts2(tm + O::xh + 16u, xin);
+            if (!kAhead) ea = lds2(tl + O::EA);
             e = vfma(ea, gin, e);
-            v = vfma(ez, xin, vfma(ev, gin, v));
+            if (!kAhead) ev = lds2(tl + O::EV);
+            v = vfma(ev, gin, v);
+            if (!kAhead) ez = lds2(tl + O::EZ);
+            v = vfma(ez, xin, v);
         }
         // true g, then true x
 #pragma unroll
@@ -741,17 +784,17 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
             e = cmul(al[j], e);
             g[j] = cadd(g[j], e);
         }
-        const double2 ck = lds2(sm + O::ck + 16u * (unsigned)k);
 #pragma unroll
         for (int j = L - 1; j >= 0; --j) {
-            v = vfma(mw[j], v, (j < kMaxPad && j < x.npad) ? c2(0.0, 0.0) : g[j]);
+            v = vfma(mw[j], v, (j < kMaxPad && j < npad) ? c2(0.0, 0.0) : g[j]);
             g[j] = v;
         }
+        const double2 ck = lds2(sm + O::ck + 16u * (unsigned)k);
         if (l == 0) {
             // x of row R1 + 1 is the entry from below; x of row R0 - 1 is
             // g_{R0-1} - w_{R0-1} x_{R0}, g_{R0-1} being the entry from above
-            sts2(tm + O::xh, cmul(ck, vfma(lds2(tm + O::wghost), v, gin)));
-            sts2(tm + O::xh + 16u, cmul(ck, xin));
+            sts2(tm + O::xh, cmul(ck, vfma(lds2(tm + O::wghost), v, lds2(tm + O::xh))));
+            sts2(tm + O::xh + 16u, cmul(ck, lds2(tm + O::xh + 16u)));
         }
         // the terms' share of the sum.  Warps k and k + half are a pair: each leaves
         // the other's half of the rows and adds its own half to what the other left.
@@ -914,18 +957,15 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
         x.npad = L - cnt;
         x.row0 = ctl->R0 + start;
     }
-    // the field above and below the lane's rows: a neighbouring lane's row or the halo
-    unsigned edges;
-    {
+    // the field above and below each lane's rows: a neighbouring lane's row or the halo
+    if (x.term == 0) {
         const int low = 32 - (n & 31), base = n >> 5, next = x.lane + 1;
         const bool top = x.lane == 0 || (base == 0 && x.lane <= low);
         const int npad_next = min(L - (next < low ? base : base + 1), L - 1);
-        edges = top ? O::misc + 16 : O::U + 16u * (unsigned)((L - 1) * 32 + x.lane - 1);
+        unsigned edges = top ? O::misc + 16 : O::U + 16u * (unsigned)((L - 1) * 32 + x.lane - 1);
         edges |= (x.lane == 31 ? O::misc + 32 : O::U + 16u * (unsigned)(npad_next * 32 + next)) << 16;
+        x.at<unsigned>(O::edges)[x.lane] = edges;
     }
-    // this CTA's mailbox slot in CTA `lane`
-    unsigned raddr = 0, count = 0;
-    if (x.lane < x.C) raddr = remote_addr(smem_u32(x.tm + O::mail) + 32u * (unsigned)x.c, (unsigned)x.lane);
 
     // steps: two of 1/(1-X), one of the ip=2 operator (first output, at r = dr:
     // cupyram.py:703), then nr of the march
@@ -971,7 +1011,7 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
                 if (tlc < ctl->nvr) out = tlc;
                 ++tlc;
             }
-            reg_step<L>(a, x, na, al, mw, edges, raddr, count, out);
+            reg_step<L>(a, x, na, al, mw, q, out);
         }
     }
     if (threadIdx.x == 0 && ctl->dead) atomicOr(a.flags + ctl->rid, 2);
