@@ -630,7 +630,7 @@ struct cr_engine {
     // one launch per (Pade term count) group on its own stream
     struct ColGroup {
         int cluster, terms, rows, nz_max, begin, count;  // rows: of a lane (march_reg.cu), 0: march_col.cu
-        bool policy;                                     // rays that the column policy took
+        bool policy;                                     // only rays that the column policy took
         cudaStream_t stream;
         cudaEvent_t done;
     };
@@ -696,6 +696,47 @@ cudaError_t engine_pool(int dev, cudaMemPool_t* out) {
     return cudaSuccess;
 }
 
+// Streams (with an event each) of the engines' launches, kept for the next
+// engine: creating and destroying one costs about 70 us, and an uneven batch
+// takes dozens.  At most kLanesKept idle ones per device; cr_release_cache
+// destroys them.  A lane is given back idle.
+struct StreamLane {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t done = nullptr;
+};
+constexpr size_t kLanesKept = 128;
+std::vector<StreamLane> g_lanes[kPoolDevices];
+std::mutex g_lanes_mu;
+
+cudaError_t lane_take(int dev, StreamLane* out) {
+    if (dev >= 0 && dev < kPoolDevices) {
+        std::lock_guard<std::mutex> lock(g_lanes_mu);
+        if (!g_lanes[dev].empty()) {
+            *out = g_lanes[dev].back();
+            g_lanes[dev].pop_back();
+            return cudaSuccess;
+        }
+    }
+    StreamLane l;
+    cudaError_t ce = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
+    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming);
+    if (ce != cudaSuccess && l.stream) cudaStreamDestroy(l.stream);
+    else *out = l;
+    return ce;
+}
+void lane_give(int dev, StreamLane l) {
+    if (!l.stream) return;
+    if (dev >= 0 && dev < kPoolDevices) {
+        std::lock_guard<std::mutex> lock(g_lanes_mu);
+        if (g_lanes[dev].size() < kLanesKept) {
+            g_lanes[dev].push_back(l);
+            return;
+        }
+    }
+    cudaEventDestroy(l.done);
+    cudaStreamDestroy(l.stream);
+}
+
 template <typename T>
 cudaError_t dev_alloc(cr_engine* e, T** p, size_t count) {
     if (count == 0) count = 1;
@@ -721,18 +762,18 @@ void free_all(cr_engine* e) {
             if (p) cudaFreeAsync(p, e->stream);
         cudaStreamSynchronize(e->stream);
     }
-    for (auto& g : e->col_groups) {
-        if (g.done) cudaEventDestroy(g.done);
-        if (g.stream) cudaStreamDestroy(g.stream);
+    // a march that failed half way may have left work on streams that never joined
+    if (!e->marched) {
+        for (auto& g : e->col_groups)
+            if (g.stream) cudaStreamSynchronize(g.stream);
+        for (size_t i = 1; i < e->sum_streams.size(); ++i)
+            if (e->sum_streams[i]) cudaStreamSynchronize(e->sum_streams[i]);
     }
-    if (e->ev_fork) cudaEventDestroy(e->ev_fork);
-    for (size_t i = 1; i < e->sum_streams.size(); ++i)
-        if (e->sum_streams[i]) cudaStreamDestroy(e->sum_streams[i]);
-    for (auto ev : e->sum_done)
-        if (ev) cudaEventDestroy(ev);
+    for (auto& g : e->col_groups) lane_give(e->device, {g.stream, g.done});
+    for (size_t i = 1; i < e->sum_streams.size(); ++i) lane_give(e->device, {e->sum_streams[i], e->sum_done[i]});
+    lane_give(e->device, {e->stream, e->ev_fork});
     for (auto& ev : e->ev)
         if (ev) cudaEventDestroy(ev);
-    if (e->stream) cudaStreamDestroy(e->stream);
 }
 
 // Pinned staging of host-to-device copies.  A pageable cudaMemcpy is staged
@@ -941,9 +982,12 @@ cudaError_t device_pade(const std::vector<PadeJob>& jobs, std::vector<double2>& 
     pd2.assign((size_t)n * CR_MAX_NP, make_double2(0.0, 0.0));
     status.assign((size_t)n, CR_OK);
     if (n == 0) return cudaSuccess;
-    cudaStream_t st = nullptr;
-    cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    int dev = 0;
+    StreamLane lane;
+    cudaError_t ce = cudaGetDevice(&dev);
+    if (ce == cudaSuccess) ce = lane_take(dev, &lane);
     if (ce != cudaSuccess) return ce;
+    cudaStream_t st = lane.stream;
     // regions rounded up to 256 bytes: the coefficient arrays are double2 and
     // must start on a 16-byte boundary whatever the number of jobs
     auto r256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -952,10 +996,8 @@ cudaError_t device_pade(const std::vector<PadeJob>& jobs, std::vector<double2>& 
     unsigned char* d = nullptr;
     // from the engines' pool, which keeps its memory (the default pool maps and
     // unmaps it on every call)
-    int dev = 0;
     cudaMemPool_t pool = nullptr;
-    ce = cudaGetDevice(&dev);
-    if (ce == cudaSuccess) ce = engine_pool(dev, &pool);
+    ce = engine_pool(dev, &pool);
     if (ce == cudaSuccess) ce = cudaMallocFromPoolAsync((void**)&d, bj + 2 * bp + bs, pool, st);
     if (ce == cudaSuccess) {
         PadeJob* dj = (PadeJob*)d;
@@ -976,7 +1018,7 @@ cudaError_t device_pade(const std::vector<PadeJob>& jobs, std::vector<double2>& 
     }
     const cudaError_t cs = cudaStreamSynchronize(st);
     if (ce == cudaSuccess) ce = cs;
-    cudaStreamDestroy(st);
+    lane_give(dev, lane);
     return ce;
 }
 
@@ -1587,7 +1629,6 @@ int cr_create(const cr_batch* b, cr_engine** out) {
             }
         std::stable_sort(cord.begin(), cord.end(), [&](int x, int y) {
             const int tx = terms_of(x), ty = terms_of(y);
-            if (is_col[(size_t)x] != is_col[(size_t)y]) return is_col[(size_t)x] > is_col[(size_t)y];
             if (tx != ty) return tx > ty;
             if (lrows[(size_t)x] != lrows[(size_t)y]) return lrows[(size_t)x] > lrows[(size_t)y];
             if (csize[(size_t)x] != csize[(size_t)y]) return csize[(size_t)x] > csize[(size_t)y];
@@ -1614,12 +1655,14 @@ int cr_create(const cr_batch* b, cr_engine** out) {
             size_t end = q;
             const int terms = terms_of(cord[q]);
             const int cluster = csize[(size_t)cord[q]], rows = lrows[(size_t)cord[q]];
-            const char policy = is_col[(size_t)cord[q]];
+            bool policy = true;  // a launch with any of the batch's other rays is not the policy's
             int nz_max = 0;
-            while (end < cord.size() && is_col[(size_t)cord[end]] == policy && terms_of(cord[end]) == terms && csize[(size_t)cord[end]] == cluster &&
-                   lrows[(size_t)cord[end]] == rows)
+            while (end < cord.size() && terms_of(cord[end]) == terms && csize[(size_t)cord[end]] == cluster &&
+                   lrows[(size_t)cord[end]] == rows) {
+                policy = policy && is_col[(size_t)cord[end]];
                 nz_max = std::max(nz_max, b->rays[cord[end++]].nz);
-            e->col_groups.push_back({cluster, terms, rows, nz_max, (int)q, (int)(end - q), policy != 0, nullptr, nullptr});
+            }
+            e->col_groups.push_back({cluster, terms, rows, nz_max, (int)q, (int)(end - q), policy, nullptr, nullptr});
             q = end;
         }
         // the groups with the longest marches are launched first
@@ -1705,7 +1748,12 @@ int cr_create(const cr_batch* b, cr_engine** out) {
     e->pool.assign(b->pool, b->pool + b->pool_len);
 
     cudaError_t ce = cudaGetDevice(&e->device);
-    if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
+    if (ce == cudaSuccess) {
+        StreamLane l;
+        ce = lane_take(e->device, &l);
+        e->stream = l.stream;
+        e->ev_fork = l.done;
+    }
     for (auto& ev : e->ev)
         if (ce == cudaSuccess) ce = cudaEventCreate(&ev);
     if (ce == cudaSuccess) ce = dev_alloc(e, &e->d_rays, e->rays.size());
@@ -1737,7 +1785,6 @@ int cr_create(const cr_batch* b, cr_engine** out) {
         if (ce == cudaSuccess) ce = dev_alloc(e, &e->d_pfc, e->pfc.size());
         if (ce == cudaSuccess) ce = dev_alloc(e, &e->d_pfcinf, e->pfcinf.size());
         if (ce == cudaSuccess && !e->col_ray.empty()) ce = dev_alloc(e, &e->d_col_ray, e->col_ray.size());
-        if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming);
         {
             // one stream per run of equal lanes per ray (the first is the engine's)
             int runs = 0;
@@ -1745,14 +1792,19 @@ int cr_create(const cr_batch* b, cr_engine** out) {
             e->sum_streams.assign((size_t)std::max(runs, 1), nullptr);
             e->sum_done.assign(e->sum_streams.size(), nullptr);
             e->sum_streams[0] = e->stream;
-            for (size_t i = 1; i < e->sum_streams.size(); ++i)
-                if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->sum_streams[i], cudaStreamNonBlocking);
-            for (auto& ev : e->sum_done)
-                if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+            for (size_t i = 1; i < e->sum_streams.size() && ce == cudaSuccess; ++i) {
+                StreamLane l;
+                ce = lane_take(e->device, &l);
+                e->sum_streams[i] = l.stream;
+                e->sum_done[i] = l.done;
+            }
         }
         for (auto& g : e->col_groups) {
-            if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking);
-            if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming);
+            if (ce != cudaSuccess) break;
+            StreamLane l;
+            ce = lane_take(e->device, &l);
+            g.stream = l.stream;
+            g.done = l.done;
         }
     }
     if (ce == cudaSuccess) ce = dev_alloc(e, &e->d_tll, (size_t)e->line_len);
@@ -2293,6 +2345,14 @@ int cr_release_cache(void) {
             set_global_error("cr_release_cache: %s", cudaGetErrorString(ce));
             return CR_ECUDA;
         }
+    }
+    std::lock_guard<std::mutex> lanes(g_lanes_mu);
+    for (int d = 0; d < kPoolDevices; ++d) {
+        for (const StreamLane& l : g_lanes[d]) {
+            cudaEventDestroy(l.done);
+            cudaStreamDestroy(l.stream);
+        }
+        g_lanes[d].clear();
     }
     return CR_OK;
 }

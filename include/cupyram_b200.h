@@ -136,9 +136,9 @@ typedef struct cr_stats {
     int32_t n_tiles;
     int64_t device_bytes;     /* device memory held by the engine               */
     int32_t column_rays;      /* rays that the column policy took out of the batch */
-    int32_t column_launches;  /* cluster launches of the last cr_march for them;
-                                 in complex128 the batch's other rays march on
-                                 clusters too (kernel_launches counts all)       */
+    int32_t column_launches;  /* cluster launches of the last cr_march that held
+                                 only such rays; in complex128 the batch's other
+                                 rays march on clusters too                      */
     int32_t queue_ctas;       /* CTAs of the persistent batched launch (0: none,
                                  or one launch per lanes-per-ray value)        */
     int32_t precision_used;   /* enum cr_precision the march runs in: the
