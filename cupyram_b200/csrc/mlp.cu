@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 
@@ -565,11 +566,93 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, float* v) {
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(u[j]);
 }
 
-template <int EPI, int BN, int ST>
-__global__ void __launch_bounds__(kUThreads)
-    gemm_tn_tile(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                 const __grid_constant__ CUtensorMap mapO, const __grid_constant__ CUtensorMap mapM, int K,
-                 const float* __restrict__ bias, int* err) {
+// The MMAs of one stage (128 rows x 64 of A, the idesc's columns x 64 of B), by one thread.
+__device__ __forceinline__ void mma_stage(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t idesc, bool first) {
+#pragma unroll
+    for (int k = 0; k < UBK / 16; ++k) {
+        const uint64_t da = umma_desc_sw128(sa + k * 32), db = umma_desc_sw128(sb + k * 32);
+        const uint32_t accum = (!first || k > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            :
+            : "r"(acc), "l"(da), "l"(db), "r"(idesc), "r"(accum)
+            : "memory");
+    }
+}
+// The barrier completes once every MMA issued so far has.
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+
+// The tensor maps and bias of up to G contractions of one shape.
+constexpr int kMaxGroup = 4;
+template <int G>
+struct TileMaps {
+    CUtensorMap a[G], b[G], o[G], m[1];  // m: the mask, of single contractions
+    const float* bias[G];
+};
+// 32 accumulator columns (of this lane's row) through bias (32 values in shared
+// memory), ReLU or mask (the row's 64-byte half h of a swizzled block), into
+// the lane's words of the output: 32 of f32, 16 of bf16.
+template <int EPI>
+__device__ __forceinline__ void epi_columns(uint32_t acc, const float* sbias, const unsigned char* mask_row, int row,
+                                            int h, uint32_t* w) {
+    float v[32];
+    tmem_ld32(acc, v);
+    if (EPI == CR_MLP_EPI_BIAS_RELU_BF16 || EPI == CR_MLP_EPI_BIAS_F32) {
+        const float4* b4 = reinterpret_cast<const float4*>(sbias);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float4 b = b4[j];
+            v[4 * j] += b.x;
+            v[4 * j + 1] += b.y;
+            v[4 * j + 2] += b.z;
+            v[4 * j + 3] += b.w;
+        }
+    }
+    if (EPI == CR_MLP_EPI_BIAS_RELU_BF16) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
+    }
+    if (EPI == CR_MLP_EPI_RELU_MASK_BF16) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint4 m = *reinterpret_cast<const uint4*>(mask_row + (((4 * h + j) ^ (row & 7)) << 4));
+            const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mm[q]));
+                v[8 * j + 2 * q] = f.x > 0.f ? v[8 * j + 2 * q] : 0.f;
+                v[8 * j + 2 * q + 1] = f.y > 0.f ? v[8 * j + 2 * q + 1] : 0.f;
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        if (!epi_bf16<EPI>()) {
+            w[j] = __float_as_uint(v[j]);
+        } else if ((j & 1) == 0) {
+            const __nv_bfloat162 p = __floats2bfloat162_rn(v[j], v[j + 1]);
+            w[j / 2] = *reinterpret_cast<const uint32_t*>(&p);
+        }
+    }
+}
+// A lane's 128 bytes into its row of a 32-row piece, in the output map's swizzle.
+__device__ __forceinline__ void put_row(unsigned char* piece, int lane, const uint32_t (&w)[32]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint4*>(piece + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+            make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+}
+
+template <int EPI, int BN, int ST, int G>
+__global__ void __launch_bounds__(kUThreads) gemm_tn_tile(const __grid_constant__ TileMaps<G> t, int K, int* err) {
+    const int group = G > 1 ? blockIdx.z : 0;
+    const CUtensorMap &mapA = t.a[group], &mapB = t.b[group], &mapO = t.o[group], &mapM = t.m[0];
+    const float* bias = t.bias[group];
     using T = TileGemm<EPI, BN, ST>;
     constexpr bool kMasked = EPI == CR_MLP_EPI_RELU_MASK_BF16;
     constexpr bool kBias = EPI == CR_MLP_EPI_BIAS_RELU_BF16 || EPI == CR_MLP_EPI_BIAS_F32;
@@ -634,27 +717,10 @@ __global__ void __launch_bounds__(kUThreads)
             ok &= mbar_wait(&full[st], (kt / ST) & 1);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t sa = smem_u32(tA(st)), sb = smem_u32(tB(st));
-#pragma unroll
-            for (int k = 0; k < UBK / 16; ++k) {
-                const uint64_t da = umma_desc_sw128(sa + k * 32), db = umma_desc_sw128(sb + k * 32);
-                const uint32_t acc = (kt > 0 || k > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                    :
-                    : "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&empty[st]))
-                         : "memory");
+            mma_stage(tmem, smem_u32(tA(st)), smem_u32(tB(st)), idesc, kt == 0);
+            mma_commit(&empty[st]);
         }
-        // the accumulator is complete once every MMA issued so far is
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                         smem_u32(done))
-                     : "memory");
+        mma_commit(done);  // the accumulator is complete
     }
     __syncwarp();
     ok &= mbar_wait(done, 0);
@@ -679,58 +745,15 @@ __global__ void __launch_bounds__(kUThreads)
         for (int c = 0; c < BN / kCols; ++c) {
             uint32_t w[32];  // the lane's 128 bytes
 #pragma unroll
-            for (int h = 0; h < kCols / 32; ++h) {
-                float v[32];
-                tmem_ld32(acc + (uint32_t)(c * kCols + 32 * h), v);
-                if (kBias) {
-                    const float4* b4 = reinterpret_cast<const float4*>(sbias + c * kCols + 32 * h);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float4 b = b4[j];
-                        v[4 * j] += b.x;
-                        v[4 * j + 1] += b.y;
-                        v[4 * j + 2] += b.z;
-                        v[4 * j + 3] += b.w;
-                    }
-                }
-                if (EPI == CR_MLP_EPI_BIAS_RELU_BF16) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
-                }
-                if (kMasked) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int ch = 4 * h + j;
-                        const uint4 m = *reinterpret_cast<const uint4*>(masks + c * UBM * 128 + row * 128 +
-                                                                       ((ch ^ (row & 7)) << 4));
-                        const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mm[q]));
-                            v[8 * j + 2 * q] = f.x > 0.f ? v[8 * j + 2 * q] : 0.f;
-                            v[8 * j + 2 * q + 1] = f.y > 0.f ? v[8 * j + 2 * q + 1] : 0.f;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    if (!epi_bf16<EPI>()) {
-                        w[j] = __float_as_uint(v[j]);
-                    } else if ((j & 1) == 0) {
-                        const __nv_bfloat162 p = __floats2bfloat162_rn(v[j], v[j + 1]);
-                        w[16 * h + j / 2] = *reinterpret_cast<const uint32_t*>(&p);
-                    }
-                }
-            }
+            for (int h = 0; h < kCols / 32; ++h)
+                epi_columns<EPI>(acc + (uint32_t)(c * kCols + 32 * h), sbias + c * kCols + 32 * h,
+                                 masks + c * UBM * 128 + row * 128, row, h, w + 16 * h);
             unsigned char* piece = stg + (c & 1) * 4096;
             if (c >= 2) {  // the copy that read this piece two turns ago is done with it
                 if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                 __syncwarp();
             }
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<uint4*>(piece + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                    make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+            put_row(piece, lane, w);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) tma_store_2d(&mapO, bn + c * kCols, bm + warp * 32, piece);
@@ -1039,7 +1062,8 @@ int gemm_feed() {
 }
 
 // ---------------------------------------------------------------------------
-// Persistent TMA-fed tcgen05 contraction with the epilogue overlapped.
+// Persistent contraction with the epilogue overlapped, for outputs of many
+// blocks.
 //
 // One CTA per SM walks the output blocks (128 x 256) in a static round
 // robin.  Six warps:
@@ -1049,25 +1073,31 @@ int gemm_feed() {
 //     each stage to its "empty" barrier and each finished block to its
 //     accumulator's "full" barrier;
 //   * warps 2..5: the epilogue, one TMEM lane quadrant each (quadrant =
-//     warp mod 4), reading block i's accumulator while the MMAs of block i+1
-//     run in the other one, then releasing it on its "empty" barrier.
+//     warp mod 4): gemm_tn_tile's pieces and bulk stores of block i, while the
+//     MMAs of block i + 1 run in the other accumulator.  Reading the last
+//     columns releases the accumulator on its "empty" barrier.
 // Every wait is bounded; a role that gives up stops, the CTA sets *err, and
 // the output is incomplete.
+//
+// 8192 x 8192 x 512 into f32: 78 us (blocks of 256 columns by gemm_tn_tile,
+// two CTAs of two stages on an SM: 91), 48 KB a K-tile and SM from L2, 10 TB/s.
 // ---------------------------------------------------------------------------
 constexpr int kPStages = 4;
 constexpr int kPThreads = 192;
-constexpr size_t kPSmem = (size_t)kPStages * kUStage + (size_t)4 * 32 * 33 * 4 + 1024 + 512;
+constexpr size_t kPSmem = (size_t)kPStages * kUStage + 4 * 8192 + 4 * 64 * sizeof(float) + 1024 + 256;
+static_assert(kPSmem <= 227 * 1024, "one CTA's shared memory");
 
 template <int EPI>
-__global__ void __launch_bounds__(kPThreads, 1) gemm_tn_persistent(const __grid_constant__ CUtensorMap mapA,
-                                                                   const __grid_constant__ CUtensorMap mapB, int M,
-                                                                   int N, int K, EpiArgs e, int* err) {
+__global__ void __launch_bounds__(kPThreads, 1)
+    gemm_tn_persistent(const __grid_constant__ TileMaps<1> t, int M, int N, int K, int* err) {
+    constexpr bool kBias = EPI == CR_MLP_EPI_BIAS_RELU_BF16 || EPI == CR_MLP_EPI_BIAS_F32;
     extern __shared__ __align__(1024) unsigned char usmem[];
     unsigned char* base = (unsigned char*)(((uintptr_t)usmem + 1023) & ~(uintptr_t)1023);
     auto tA = [&](int st) { return base + st * kUStage; };
     auto tB = [&](int st) { return base + st * kUStage + kUTileA; };
-    float* stg_all = reinterpret_cast<float*>(base + kPStages * kUStage);
-    uint64_t* full = (uint64_t*)(base + kPStages * kUStage + 4 * 32 * 33 * 4);
+    unsigned char* stg_all = base + kPStages * kUStage;
+    float* sbias_all = (float*)(stg_all + 4 * 8192);
+    uint64_t* full = (uint64_t*)(sbias_all + 4 * 64);
     uint64_t* empty = full + kPStages;
     uint64_t* acc_full = empty + kPStages;   // [2]
     uint64_t* acc_empty = acc_full + 2;      // [2]
@@ -1108,8 +1138,8 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tn_persistent(const __grid_
                     if (g >= kPStages) ok &= mbar_wait(&empty[st], ((g / kPStages) - 1) & 1);
                     if (!ok) break;
                     mbar_expect_tx(&full[st], (unsigned)kUStage);
-                    tma_load_2d(tA(st), &mapA, kt * UBK, bm, &full[st]);
-                    tma_load_2d(tB(st), &mapB, kt * UBK, bn, &full[st]);
+                    tma_load_2d(tA(st), &t.a[0], kt * UBK, bm, &full[st]);
+                    tma_load_2d(tB(st), &t.b[0], kt * UBK, bn, &full[st]);
                     issued = g + 1;
                 }
             }
@@ -1129,67 +1159,57 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tn_persistent(const __grid_
                     ok &= mbar_wait(&full[st], (g / kPStages) & 1);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t sa = smem_u32(tA(st)), sb = smem_u32(tB(st));
-#pragma unroll
-                    for (int k = 0; k < UBK / 16; ++k) {
-                        const uint64_t da = umma_desc_sw128(sa + k * 32), db = umma_desc_sw128(sb + k * 32);
-                        const uint32_t accum = (kt > 0 || k > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\t"
-                            "setp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                            :
-                            : "r"(acc_addr), "l"(da), "l"(db), "r"(kUIdesc), "r"(accum)
-                            : "memory");
-                    }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     smem_u32(&empty[st]))
-                                 : "memory");
+                    mma_stage(acc_addr, smem_u32(tA(st)), smem_u32(tB(st)), kUIdesc, kt == 0);
+                    mma_commit(&empty[st]);
                 }
                 if (!ok) break;
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&acc_full[a]))
-                             : "memory");
+                mma_commit(&acc_full[a]);
             }
         }
     } else {
         // epilogue: TMEM lane quadrant q = warp mod 4 holds rows 32q..32q+31
+        constexpr int kCols = epi_bf16<EPI>() ? 64 : 32;  // columns of a piece: 128 bytes a row
         const int q = warp & 3;
-        float* stg = stg_all + (warp - 2) * 32 * 33;
-        int i = 0;
+        unsigned char* stg = stg_all + (warp - 2) * 8192;  // two pieces of 4 KB
+        float* sbias = sbias_all + (warp - 2) * 64;
+        int i = 0, n = 0;  // blocks, pieces
         for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
             const int a = i & 1;
             const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * UBN;
             ok &= mbar_wait(&acc_full[a], (i / 2) & 1);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * UBN);
 #pragma unroll 1
-            for (int cc = 0; cc < UBN; cc += 32) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t v[16];
-                    const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * UBN + cc + 16 * h);
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-                        "%15}, [%16];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                          "=r"(v[14]), "=r"(v[15])
-                        : "r"(ta));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) stg[lane * 33 + 16 * h + j] = __uint_as_float(v[j]);
+            for (int c = 0; c < UBN / kCols; ++c, ++n) {
+                if (kBias) {
+                    __syncwarp();
+                    for (int j = lane; j < kCols; j += 32) sbias[j] = t.bias[0][bn + c * kCols + j];
+                    __syncwarp();
                 }
+                uint32_t w[32];  // the lane's 128 bytes
+#pragma unroll
+                for (int h = 0; h < kCols / 32; ++h)
+                    epi_columns<EPI>(acc + (uint32_t)(c * kCols + 32 * h), sbias + 32 * h, nullptr, lane, h, w + 16 * h);
+                if (c == UBN / kCols - 1) {
+                    // this warp's reads of the accumulator are done: release it to the MMAs
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[a])) : "memory");
+                }
+                unsigned char* piece = stg + (n & 1) * 4096;
+                if (n >= 2) {  // the copy that read this piece two turns ago is done with it
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    __syncwarp();
+                }
+                put_row(piece, lane, w);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-#pragma unroll 4
-                for (int r = 0; r < 32; ++r) store1<EPI>(e, bm + q * 32 + r, bn + cc + lane, stg[r * 33 + lane]);
-                __syncwarp();
+                if (lane == 0) tma_store_2d(&t.o[0], bn + c * kCols, bm + q * 32, piece);
             }
-            // this warp's reads of the accumulator are done: release it to the MMAs
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[a])) : "memory");
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     __syncwarp();
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
@@ -1202,6 +1222,185 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tn_persistent(const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * UBN));
+}
+
+// ---------------------------------------------------------------------------
+// Output layers of an ensemble with the statistics in the epilogue.
+//
+// Each member's outputs were written (134 MB for 4096 requests), read again by
+// ensemble_stats and thrown away: 4 x 54 us of contractions and 127 us of
+// statistics for 4000 requests and four members.  Here a CTA accumulates the
+// same 128 x 128 block of every member side by side in tensor memory (M x 128
+// of the 512 columns; two members leave room for two blocks), and the epilogue
+// turns them into mean and spread in registers: only the results leave (343 ->
+// 297 us), and the hidden layers of all members share a launch each (160 -> 47 us
+// over three layers: 256 CTAs a launch left the last of two waves half empty).  Roles
+// as in gemm_tn_persistent, with eight epilogue warps (a lane quadrant and
+// half of the columns each).  Every value sees ensemble_stats' operations in
+// its order.
+// ---------------------------------------------------------------------------
+struct EnsembleArgs {
+    CUtensorMap a[kMaxGroup], b[kMaxGroup], mean, spread;
+    const float* bias[kMaxGroup];
+    float scale, mid, lo, hi;
+};
+constexpr int kEBN = 128, kEStage = kUTileA + kEBN * UBK * 2, kEStages = 4;
+constexpr int kEWarps = 8;  // of the epilogue
+constexpr int kEThreads = 64 + 32 * kEWarps;
+constexpr size_t kESmem = (size_t)kEStages * kEStage + kEWarps * (8192 + kMaxGroup * 32 * sizeof(float)) + 1024 + 256;
+
+template <int M>
+__global__ void __launch_bounds__(kEThreads, 1)
+    ensemble_tile(const __grid_constant__ EnsembleArgs t, int rows, int N, int K, int* err) {
+    static_assert(M >= 2 && M <= kMaxGroup, "members side by side in tensor memory");
+    constexpr int kBufs = M * kEBN * 2 <= 512 ? 2 : 1, kColumns = 512;
+    constexpr uint32_t idesc =
+        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kEBN >> 3) << 17) | ((uint32_t)(UBM >> 4) << 24);
+    extern __shared__ __align__(1024) unsigned char usmem[];
+    unsigned char* base = (unsigned char*)(((uintptr_t)usmem + 1023) & ~(uintptr_t)1023);
+    auto tA = [&](int st) { return base + st * kEStage; };
+    auto tB = [&](int st) { return base + st * kEStage + kUTileA; };
+    unsigned char* stg_all = base + kEStages * kEStage;
+    float* sbias_all = (float*)(stg_all + kEWarps * 8192);
+    uint64_t* full = (uint64_t*)(sbias_all + kEWarps * kMaxGroup * 32);
+    uint64_t* empty = full + kEStages;
+    uint64_t* acc_full = empty + kEStages;      // [kBufs]
+    uint64_t* acc_empty = acc_full + kBufs;     // [kBufs]
+    uint32_t* taddr_s = (uint32_t*)(acc_empty + kBufs);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nk = K / UBK, nbm = rows / UBM, nblocks = nbm * (N / kEBN);
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(taddr_s)),
+                     "r"(kColumns));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    if (tid == 32) {
+        for (int s = 0; s < kEStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < kBufs; ++a) {
+            mbar_init(&acc_full[a], 1);
+            mbar_init(&acc_empty[a], kEWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *taddr_s;
+    bool ok = true;
+    int issued = 0;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int g = 0;
+            for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x) {
+                const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * kEBN;
+                for (int k = 0; k < M && ok; ++k)
+                    for (int kt = 0; kt < nk && ok; ++kt, ++g) {
+                        const int st = g % kEStages;
+                        if (g >= kEStages) ok &= mbar_wait(&empty[st], ((g / kEStages) - 1) & 1);
+                        if (!ok) break;
+                        mbar_expect_tx(&full[st], (unsigned)kEStage);
+                        tma_load_2d(tA(st), &t.a[k], kt * UBK, bm, &full[st]);
+                        tma_load_2d(tB(st), &t.b[k], kt * UBK, bn, &full[st]);
+                        issued = g + 1;
+                    }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int g = 0, i = 0;
+            for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
+                const int a = i % kBufs;
+                if (i >= kBufs) ok &= mbar_wait(&acc_empty[a], ((i / kBufs) - 1) & 1);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int k = 0; k < M && ok; ++k)
+                    for (int kt = 0; kt < nk && ok; ++kt, ++g) {
+                        const int st = g % kEStages;
+                        ok &= mbar_wait(&full[st], (g / kEStages) & 1);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        mma_stage(tmem + (uint32_t)((a * M + k) * kEBN), smem_u32(tA(st)), smem_u32(tB(st)), idesc,
+                                  kt == 0);
+                        mma_commit(&empty[st]);
+                    }
+                if (!ok) break;
+                mma_commit(&acc_full[a]);
+            }
+        }
+    } else {
+        const int q = warp & 3, half = (warp - 2) >> 2;
+        unsigned char* stg = stg_all + (warp - 2) * 8192;  // a piece of the mean, one of the spread
+        float* sbias = sbias_all + (warp - 2) * kMaxGroup * 32;
+        const float inv = 1.f / (float)M;
+        int i = 0, n = 0;
+        for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
+            const int a = i % kBufs;
+            const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * kEBN;
+            ok &= mbar_wait(&acc_full[a], (i / kBufs) & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+            for (int c = 2 * half; c < 2 * half + 2; ++c, ++n) {
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < M; ++k) sbias[k * 32 + lane] = t.bias[k][bn + c * 32 + lane];
+                __syncwarp();
+                float x[M][32];
+#pragma unroll
+                for (int k = 0; k < M; ++k)
+                    tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((a * M + k) * kEBN + c * 32), x[k]);
+                if (c == 2 * half + 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[a])) : "memory");
+                }
+                uint32_t mean[32], spread[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    float s = 0.f, d = 0.f;
+#pragma unroll
+                    for (int k = 0; k < M; ++k) {
+                        x[k][j] = member_tl(x[k][j] + sbias[k * 32 + j], t.scale, t.mid, t.lo, t.hi);
+                        s += x[k][j];
+                    }
+                    s *= inv;
+#pragma unroll
+                    for (int k = 0; k < M; ++k) d = fmaf(x[k][j] - s, x[k][j] - s, d);
+                    mean[j] = __float_as_uint(s);
+                    spread[j] = __float_as_uint(sqrtf(d * inv));
+                }
+                if (n > 0) {  // the copies of the last pieces have read them
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    __syncwarp();
+                }
+                put_row(stg, lane, mean);
+                put_row(stg + 4096, lane, spread);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&t.mean, bn + c * 32, bm + q * 32, stg);
+                    tma_store_2d(&t.spread, bn + c * 32, bm + q * 32, stg + 4096);
+                }
+            }
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    __syncwarp();
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    if (!ok && warp == 0 && lane == 0) {
+        for (int g = issued - 1; g >= 0 && g >= issued - kEStages; --g)
+            mbar_wait(&full[g % kEStages], (g / kEStages) & 1);
+    }
+    if (!ok && tid == 0) atomicExch(err, 1);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kColumns));
 }
 
 using crk::encode_tiled;
@@ -1242,33 +1441,80 @@ struct TileOperands {
     int M, N, K, lda, ldb;
 };
 
-template <int EPI, int BN, int ST>
-cudaError_t launch_tile(const TileOperands& o, const EpiArgs& e, int* err, cudaStream_t st) {
+// G equal contractions (o and e of each) by gemm_tn_tile.
+template <int EPI, int BN, int ST, int G>
+cudaError_t launch_tile(const TileOperands* o, const EpiArgs* e, int* err, cudaStream_t st) {
     using T = TileGemm<EPI, BN, ST>;
-    CUtensorMap ma, mb, mo, mm;
-    if (!operand_map(&ma, o.A, o.M, o.K, o.lda, UBM) || !operand_map(&mb, o.B, o.N, o.K, o.ldb, BN) ||
-        !tile_map(&mo, e.out, epi_bf16<EPI>(), o.M, o.N, e.ldo, 32))
-        return cudaErrorUnknown;
-    mm = mo;
-    if (T::kMask && !tile_map(&mm, e.mask, true, o.M, o.N, e.ldm, UBM)) return cudaErrorUnknown;
-    const cudaError_t ce = cudaFuncSetAttribute(gemm_tn_tile<EPI, BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)T::smem);
+    TileMaps<G> t;
+    for (int g = 0; g < G; ++g) {
+        if (!operand_map(&t.a[g], o[g].A, o[g].M, o[g].K, o[g].lda, UBM) ||
+            !operand_map(&t.b[g], o[g].B, o[g].N, o[g].K, o[g].ldb, BN) ||
+            !tile_map(&t.o[g], e[g].out, epi_bf16<EPI>(), o[g].M, o[g].N, e[g].ldo, 32))
+            return cudaErrorUnknown;
+        t.bias[g] = e[g].bias;
+    }
+    t.m[0] = t.o[0];
+    if (T::kMask && !tile_map(&t.m[0], e[0].mask, true, o[0].M, o[0].N, e[0].ldm, UBM)) return cudaErrorUnknown;
+    auto* f = gemm_tn_tile<EPI, BN, ST, G>;
+    const cudaError_t ce = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem);
     if (ce != cudaSuccess) return ce;
-    gemm_tn_tile<EPI, BN, ST><<<dim3(o.N / BN, o.M / UBM), kUThreads, T::smem, st>>>(ma, mb, mo, mm, o.K, e.bias, err);
+    f<<<dim3(o[0].N / BN, o[0].M / UBM, G), kUThreads, T::smem, st>>>(t, o[0].K, err);
     return cudaGetLastError();
 }
 
-// The widest block that still gives every SM of the device work (148 on a
-// B200; two blocks each at 256 columns, whose two CTAs share an SM).
+int sm_count() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 template <int EPI>
-cudaError_t launch_tile_n(const TileOperands& o, const EpiArgs& e, int* err, cudaStream_t st) {
+cudaError_t launch_persistent(const TileOperands& o, const EpiArgs& e, int* err, cudaStream_t st) {
+    TileMaps<1> t;
+    if (!operand_map(&t.a[0], o.A, o.M, o.K, o.lda, UBM) || !operand_map(&t.b[0], o.B, o.N, o.K, o.ldb, UBN) ||
+        !tile_map(&t.o[0], e.out, epi_bf16<EPI>(), o.M, o.N, e.ldo, 32))
+        return cudaErrorUnknown;
+    t.m[0] = t.o[0];
+    t.bias[0] = e.bias;
+    auto* f = gemm_tn_persistent<EPI>;
+    const cudaError_t ce = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmem);
+    if (ce != cudaSuccess) return ce;
+    const int blocks = (o.M / UBM) * (o.N / UBN), sms = sm_count();
+    f<<<std::min(blocks, sms), kPThreads, kPSmem, st>>>(t, o.M, o.N, o.K, err);
+    return cudaGetLastError();
+}
+
+// The persistent kernel once every SM has two of its blocks (256 columns; 78 us
+// at 8192 x 8192 x 512, 91 by blocks of gemm_tn_tile), else the widest block that
+// still gives every SM work.  walk: the persistent
+// kernel at any size (a mask takes its shared memory: never there).
+template <int EPI>
+cudaError_t launch_tile_n(const TileOperands& o, const EpiArgs& e, bool walk, int* err, cudaStream_t st) {
     constexpr int kSms = 148;
     const long long rows = o.M / UBM;
     if constexpr (EPI != CR_MLP_EPI_RELU_MASK_BF16) {
-        if (rows * (o.N / 256) >= 2 * kSms) return launch_tile<EPI, 256, 2>(o, e, err, st);
+        if (walk || rows * (o.N / 256) >= 2 * kSms) return launch_persistent<EPI>(o, e, err, st);
     }
-    if (rows * (o.N / 128) >= kSms) return launch_tile<EPI, 128, 3>(o, e, err, st);
-    return launch_tile<EPI, 64, 7>(o, e, err, st);
+    if (rows * (o.N / 128) >= kSms) return launch_tile<EPI, 128, 3, 1>(&o, &e, err, st);
+    return launch_tile<EPI, 64, 7, 1>(&o, &e, err, st);
+}
+
+// G equal hidden layers (bias, ReLU, bf16) in one launch.
+template <int G>
+cudaError_t launch_hidden(const TileOperands* o, const EpiArgs* e, int* err, cudaStream_t st) {
+    constexpr int kSms = 148;
+    const long long rows = (long long)(o[0].M / UBM) * G;
+    if (rows * (o[0].N / 128) >= kSms) return launch_tile<CR_MLP_EPI_BIAS_RELU_BF16, 128, 3, G>(o, e, err, st);
+    return launch_tile<CR_MLP_EPI_BIAS_RELU_BF16, 64, 7, G>(o, e, err, st);
+}
+
+template <int M>
+cudaError_t launch_ensemble(const EnsembleArgs& t, int rows, int N, int K, int* err, cudaStream_t st) {
+    const cudaError_t ce =
+        cudaFuncSetAttribute(ensemble_tile<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kESmem);
+    if (ce != cudaSuccess) return ce;
+    ensemble_tile<M><<<std::min((rows / UBM) * (N / kEBN), sm_count()), kEThreads, kESmem, st>>>(t, rows, N, K, err);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -1312,47 +1558,22 @@ int cr_mlp_gemm_tc(int epi, const void* A, const void* B, int M, int N, int K, i
     auto b = (const __nv_bfloat16*)B;
     cudaError_t ce = cudaSuccess;
     const int feed = gemm_feed();
-    if (feed == 2) {
-        // persistent: one CTA per SM, operands by the tensor memory accelerator
-        CUtensorMap ma, mb;
-        if (!operand_map(&ma, A, M, K, lda, UBM) || !operand_map(&mb, B, N, K, ldb, UBN)) return CR_MLP_ECUDA;
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return CR_MLP_ECUDA;
-        const int blocks = (M / UBM) * (N / UBN);
-        const int ctas = blocks < sms ? blocks : sms;
-        switch (epi) {
-#define CR_PERS_CASE(E)                                                                                          \
-    case E:                                                                                                      \
-        ce = cudaFuncSetAttribute(gemm_tn_persistent<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmem); \
-        if (ce == cudaSuccess) gemm_tn_persistent<E><<<ctas, kPThreads, kPSmem, st>>>(ma, mb, M, N, K, e, err);    \
-        break;
-            CR_PERS_CASE(CR_MLP_EPI_BIAS_RELU_BF16)
-            CR_PERS_CASE(CR_MLP_EPI_BIAS_F32)
-            CR_PERS_CASE(CR_MLP_EPI_F32)
-            CR_PERS_CASE(CR_MLP_EPI_RELU_MASK_BF16)
-#undef CR_PERS_CASE
-            default: return CR_MLP_EBADSHAPE;
-        }
-        if (ce != cudaSuccess) return CR_MLP_ECUDA;
-        return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
-    }
     // outputs (and a mask) whose rows start on 16-byte boundaries leave by bulk copies
     const bool half = epi == CR_MLP_EPI_BIAS_RELU_BF16 || epi == CR_MLP_EPI_RELU_MASK_BF16;
     const bool out16 = aligned16(out) && ldo % (half ? 8 : 4) == 0;
-    if (feed == 1 && out16 && (epi != CR_MLP_EPI_RELU_MASK_BF16 || (aligned16(mask) && ldm % 8 == 0))) {
+    if (feed >= 1 && out16 && (epi != CR_MLP_EPI_RELU_MASK_BF16 || (aligned16(mask) && ldm % 8 == 0))) {
         const TileOperands o{A, B, M, N, K, lda, ldb};
+        const bool walk = feed == 2;
         switch (epi) {
-            case CR_MLP_EPI_BIAS_RELU_BF16: ce = launch_tile_n<CR_MLP_EPI_BIAS_RELU_BF16>(o, e, err, st); break;
-            case CR_MLP_EPI_BIAS_F32: ce = launch_tile_n<CR_MLP_EPI_BIAS_F32>(o, e, err, st); break;
-            case CR_MLP_EPI_F32: ce = launch_tile_n<CR_MLP_EPI_F32>(o, e, err, st); break;
-            case CR_MLP_EPI_RELU_MASK_BF16: ce = launch_tile_n<CR_MLP_EPI_RELU_MASK_BF16>(o, e, err, st); break;
+            case CR_MLP_EPI_BIAS_RELU_BF16: ce = launch_tile_n<CR_MLP_EPI_BIAS_RELU_BF16>(o, e, walk, err, st); break;
+            case CR_MLP_EPI_BIAS_F32: ce = launch_tile_n<CR_MLP_EPI_BIAS_F32>(o, e, walk, err, st); break;
+            case CR_MLP_EPI_F32: ce = launch_tile_n<CR_MLP_EPI_F32>(o, e, walk, err, st); break;
+            case CR_MLP_EPI_RELU_MASK_BF16: ce = launch_tile_n<CR_MLP_EPI_RELU_MASK_BF16>(o, e, walk, err, st); break;
             default: return CR_MLP_EBADSHAPE;
         }
         return ce == cudaSuccess ? 0 : CR_MLP_ECUDA;
     }
-    if (feed == 1) {
+    if (feed >= 1) {
         // operands by the tensor memory accelerator (tensor maps over this GPU's memory)
         CUtensorMap ma, mb;
         if (!operand_map(&ma, A, M, K, lda, UBM) || !operand_map(&mb, B, N, K, ldb, UBN)) return CR_MLP_ECUDA;
@@ -1550,6 +1771,77 @@ int cr_mlp_step(const cr_mlp_net* net, float lr, float beta1, float beta2, float
                                                                   weight_decay);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : CR_MLP_ECUDA;
+}
+
+namespace {
+// The members' networks have one shape, and every contraction is one that the
+// default tcgen05 path takes with bulk-copy epilogues.
+bool ensemble_fits(const cr_mlp_net* const* nets, int members, int batch, const void* x, int ldx, int tc,
+                   const float* mean, const float* spread) {
+    if (!tc || members < 2 || members > kMaxGroup || gemm_feed() != 1 || ldx < nets[0]->dims[0] || ldx % 8 ||
+        !aligned16(x) || !aligned16(mean) || !aligned16(spread))
+        return false;
+    const int L = nets[0]->layers;
+    for (int k = 0; k < members; ++k) {
+        if (nets[k]->layers != L || !mlp_dims_ok(nets[k], batch)) return false;
+        for (int l = 0; l <= L; ++l)
+            if (nets[k]->dims[l] != nets[0]->dims[l]) return false;
+        for (int l = 0; l < L; ++l)
+            if (nets[k]->dims[l + 1] % UBN || nets[k]->dims[l] % UBK || !nets[k]->b[l] ||
+                !aligned16(nets[k]->w16[l]) || (l > 0 && !aligned16(nets[k]->act[l])))
+                return false;
+    }
+    return true;
+}
+}  // namespace
+
+int cr_mlp_ensemble_predict(const cr_mlp_net* const* nets, int members, int batch, const void* x, int ldx,
+                            float* const* outs, int tc, float scale, float mid, float lo, float hi, float* mean,
+                            float* spread, int* err, void* stream) {
+    if (!nets || members < 1 || members > kMaxMembers || !x || !outs || !mean || !spread) return CR_MLP_EBADSHAPE;
+    for (int k = 0; k < members; ++k)
+        if (!nets[k] || !mlp_dims_ok(nets[k], batch)) return CR_MLP_EBADSHAPE;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!err || !ensemble_fits(nets, members, batch, x, ldx, tc, mean, spread)) {
+        for (int k = 0; k < members; ++k) {
+            const int rc = cr_mlp_forward(nets[k], batch, x, ldx, outs[k], tc, err, stream);
+            if (rc) return rc;
+        }
+        const long long n = (long long)batch * nets[0]->dims[nets[0]->layers];
+        return cr_mlp_ensemble_stats(outs, members, n, scale, mid, lo, hi, mean, spread, stream);
+    }
+    const int L = nets[0]->layers;
+    const int* d = nets[0]->dims;
+    cudaError_t ce = cudaSuccess;
+    for (int l = 0; l < L - 1 && ce == cudaSuccess; ++l) {
+        TileOperands o[kMaxGroup];
+        EpiArgs e[kMaxGroup];
+        for (int k = 0; k < members; ++k) {
+            o[k] = {l ? nets[k]->act[l] : x, nets[k]->w16[l], batch, d[l + 1], d[l], l ? d[l] : ldx, d[l]};
+            e[k] = {nets[k]->act[l + 1], d[l + 1], nets[k]->b[l], nullptr, 0};
+        }
+        ce = members == 2 ? launch_hidden<2>(o, e, err, st)
+                          : (members == 3 ? launch_hidden<3>(o, e, err, st) : launch_hidden<4>(o, e, err, st));
+    }
+    if (ce != cudaSuccess) return CR_MLP_ECUDA;
+    EnsembleArgs t;
+    const int K = d[L - 1], N = d[L];
+    for (int k = 0; k < members; ++k) {
+        if (!operand_map(&t.a[k], L > 1 ? nets[k]->act[L - 1] : x, batch, K, L > 1 ? K : ldx, UBM) ||
+            !operand_map(&t.b[k], nets[k]->w16[L - 1], N, K, K, kEBN))
+            return CR_MLP_ECUDA;
+        t.bias[k] = nets[k]->b[L - 1];
+    }
+    if (!tile_map(&t.mean, mean, false, batch, N, N, 32) || !tile_map(&t.spread, spread, false, batch, N, N, 32))
+        return CR_MLP_ECUDA;
+    t.scale = scale;
+    t.mid = mid;
+    t.lo = lo;
+    t.hi = hi;
+    ce = members == 2 ? launch_ensemble<2>(t, batch, N, K, err, st)
+                      : (members == 3 ? launch_ensemble<3>(t, batch, N, K, err, st)
+                                      : launch_ensemble<4>(t, batch, N, K, err, st));
+    return ce == cudaSuccess ? CR_MLP_OK : CR_MLP_ECUDA;
 }
 
 int cr_mlp_ensemble_stats(const float* const* preds, int members, long long n, float scale, float mid, float lo,

@@ -97,8 +97,11 @@ _SIGS.update({
                     ctypes.c_int, ctypes.c_float, ctypes.c_void_p],
     "cr_mlp_ensemble_stats": [ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_float,
                               ctypes.c_float, ctypes.c_float, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p],
+    "cr_mlp_ensemble_predict": [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
+                                ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                                ctypes.c_float, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p],
 })
-MAX_MEMBERS = 64  # of cr_mlp_ensemble_stats
+MAX_MEMBERS = 64  # of cr_mlp_ensemble_predict
 # Contractions with N a multiple of 256 and K of 64 run on the tcgen05 tensor
 # cores (cr_mlp_gemm_tc); the others on the mma.sync kernel (cr_mlp_gemm).
 USE_TCGEN05 = True
@@ -455,6 +458,20 @@ class Ensemble:
             losses.append(math.sqrt(mse) * TL_SCALE)
         return losses
 
+    def _predict_chunk(self, X, mean, spread):
+        B, n = X.shape[0], len(self.models)
+        nets, outs = [], []
+        for m in self.models:
+            bufs = m._buffers(B)
+            assert X.shape[1] == m.dims[0]
+            bufs[0][0] = X
+            nets.append(m._net(B, w16=m.Wb, b=m.b))
+            outs.append(bufs[1].data_ptr())
+        _ok(kernels().cr_mlp_ensemble_predict((ctypes.c_void_p * n)(*[ctypes.addressof(t) for t in nets]), n, B, _p(X),
+                                              X.stride(0), (ctypes.c_void_p * n)(*outs), int(USE_TCGEN05), TL_SCALE,
+                                              TL_MID, TL_LO, TL_HI, _p(mean), _p(spread), _p(tc_error_flag()),
+                                              _stream()), "cr_mlp_ensemble_predict")
+
     def predict(self, X, chunk=8192, check=True):
         """TL mean and spread over the members, [n, 64, 128] each (dB, float32 device tensors).
         check: synchronise and raise if a tensor-core GEMM gave up a wait (callers that
@@ -465,14 +482,10 @@ class Ensemble:
         spread = torch.empty(n, NZ_OUT * NR_OUT, device=X.device)
         for s in range(0, n, chunk):
             xb = X[s: s + chunk]
-            # every member's output stays in its own buffer until the statistics have read it
-            preds = [m.forward(xb) for m in self.models]
-            if len(preds) <= MAX_MEMBERS:
-                ptrs = (ctypes.c_void_p * len(preds))(*[p.data_ptr() for p in preds])
-                _ok(kernels().cr_mlp_ensemble_stats(ptrs, len(preds), preds[0].numel(), TL_SCALE, TL_MID, TL_LO, TL_HI,
-                                                    _p(mean[s: s + chunk]), _p(spread[s: s + chunk]), _stream()),
-                    "cr_mlp_ensemble_stats")
+            if len(self.models) <= MAX_MEMBERS:
+                self._predict_chunk(xb, mean[s: s + chunk], spread[s: s + chunk])
                 continue
+            preds = [m.forward(xb) for m in self.models]
             tl = (torch.stack(preds) * TL_SCALE + TL_MID).clamp_(TL_LO, TL_HI)
             mean[s: s + chunk] = tl.mean(0)
             spread[s: s + chunk] = tl.std(0, unbiased=False)

@@ -110,6 +110,17 @@ int cr_mlp_step(const cr_mlp_net* net, float lr, float beta1, float beta2, float
 int cr_mlp_ensemble_stats(const float* const* preds, int members, long long n, float scale, float mid, float lo,
                           float hi, float* mean, float* spread, void* stream);
 
+/* The ensemble's forward passes for x (bf16, row stride ldx) and their
+ * statistics, as cr_mlp_forward of every member and cr_mlp_ensemble_stats give
+ * them; mean and spread are [batch][dims[layers]].  nets: host array of
+ * `members` networks (w16, b and act are used).  Two to four members of one
+ * shape, all of it on the tcgen05 kernel, take one launch a hidden layer and one
+ * for the output layers with the statistics; outs[k] is then left as it was.
+ * Otherwise outs[k] (16-byte aligned) holds member k's outputs. */
+int cr_mlp_ensemble_predict(const cr_mlp_net* const* nets, int members, int batch, const void* x, int ldx,
+                            float* const* outs, int tc, float scale, float mid, float lo, float hi, float* mean,
+                            float* spread, int* err, void* stream);
+
 /* dst = BF16(src) for n values. */
 int cr_mlp_to_bf16(const float* src, void* dst, long long n, void* stream);
 

@@ -104,3 +104,32 @@ def test_ensemble_statistics(cuda_device, members, n):
     assert (spread[ok].double() - tl.std(0, unbiased=False)[ok]).abs().max() < 1e-3
     assert S.kernels().cr_mlp_ensemble_stats(ptrs, members, n - 1, 25.0, 90.0, 20.0, 150.0, S._p(mean), S._p(spread),
                                              S._stream()) != 0
+
+
+# one block per CTA, several, rings that wrap within a block, no hidden layer; 384: not the fused path
+@pytest.mark.parametrize("dims", [[128, 256], [128, 256, 512, 4096], [192 * 2, 256, 768], [128, 384, 256]])
+@pytest.mark.parametrize("members", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("batch", [128, 2432])
+def test_ensemble_predict_matches_forward_and_statistics(cuda_device, dims, members, batch):
+    import torch
+    from cupyram_b200 import surrogate as S
+    models = [S.MLP(dims, seed=k) for k in range(members)]
+    g = torch.Generator(device="cuda").manual_seed(2)
+    for m in models:
+        for b in m.b:
+            b.copy_(torch.randn(b.shape, generator=g, device="cuda"))
+    X = torch.randn(batch, dims[0], generator=g, device="cuda").to(torch.bfloat16)
+    n = batch * dims[-1]
+    S.tc_error_flag().zero_()
+    mean, spread, m0, s0 = (torch.full((batch, dims[-1]), float("nan"), device="cuda") for _ in range(4))
+    e = S.Ensemble.__new__(S.Ensemble)
+    e.models = models
+    e._predict_chunk(X, mean, spread)
+    preds = [m.forward(X) for m in models]
+    ptrs = (ctypes.c_void_p * members)(*[p.data_ptr() for p in preds])
+    assert S.kernels().cr_mlp_ensemble_stats(ptrs, members, n, S.TL_SCALE, S.TL_MID, S.TL_LO, S.TL_HI, S._p(m0),
+                                             S._p(s0), S._stream()) == 0
+    # the same sums over K in the same order; at most the statistics' own FP32 rounding of values up to 150
+    assert (mean - m0).abs().max() <= 150 * 2 ** -22
+    assert (spread - s0).abs().max() <= 1e-3
+    assert int(S.tc_error_flag().item()) == 0
