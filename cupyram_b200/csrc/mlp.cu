@@ -648,6 +648,13 @@ __device__ __forceinline__ void put_row(unsigned char* piece, int lane, const ui
             make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
 }
 
+// 32 bytes of a lane: a whole sector of its row.
+__device__ __forceinline__ void store_sector(void* p, const uint32_t* w) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
 template <int EPI, int BN, int ST, int G>
 __global__ void __launch_bounds__(kUThreads) gemm_tn_tile(const __grid_constant__ TileMaps<G> t, int K, int* err) {
     const int group = G > 1 ? blockIdx.z : 0;
@@ -988,8 +995,10 @@ struct Members {
     const float* out[kMaxMembers];
 };
 __device__ __forceinline__ float member_tl(float x, float scale, float mid, float lo, float hi) {
-    const float t = __fadd_rn(__fmul_rn(x, scale), mid);
-    return t < lo ? lo : (t > hi ? hi : t);  // a NaN stays
+    float t = __fadd_rn(__fmul_rn(x, scale), mid);
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(lo));  // a NaN stays
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(t) : "f"(hi));
+    return t;
 }
 template <int M>  // members held in registers; 0: any number, read twice
 __global__ void __launch_bounds__(256) ensemble_stats(const __grid_constant__ Members p, int members, long long n4,
@@ -1079,8 +1088,11 @@ int gemm_feed() {
 // Every wait is bounded; a role that gives up stops, the CTA sets *err, and
 // the output is incomplete.
 //
-// 8192 x 8192 x 512 into f32: 78 us (blocks of 256 columns by gemm_tn_tile,
-// two CTAs of two stages on an SM: 91), 48 KB a K-tile and SM from L2, 10 TB/s.
+// 8192 x 8192 x 512 into f32: 79 us (blocks of 256 columns by gemm_tn_tile, two
+// CTAs of two stages on an SM: 91).  Without its stores it takes 50 us (38 the
+// loads alone), with a K of 64 its 268 MB take 54 (a fill: 39); the two share the
+// shared memory's bandwidth.  Eight epilogue warps (79 us), 32-byte stores straight
+// from registers (88) and other walks over the blocks (80-81) gained nothing.
 // ---------------------------------------------------------------------------
 constexpr int kPStages = 4;
 constexpr int kPThreads = 192;
@@ -1232,22 +1244,34 @@ __global__ void __launch_bounds__(kPThreads, 1)
 // statistics for 4000 requests and four members.  Here a CTA accumulates the
 // same 128 x 128 block of every member side by side in tensor memory (M x 128
 // of the 512 columns; two members leave room for two blocks), and the epilogue
-// turns them into mean and spread in registers: only the results leave (343 ->
-// 297 us), and the hidden layers of all members share a launch each (160 -> 47 us
-// over three layers: 256 CTAs a launch left the last of two waves half empty).  Roles
-// as in gemm_tn_persistent, with eight epilogue warps (a lane quadrant and
-// half of the columns each).  Every value sees ensemble_stats' operations in
+// turns them into mean and spread in registers: only the results leave, by whole
+// 32-byte sectors of a lane's row (343 -> 264 us; the contractions' part alone is
+// 190), and the hidden layers of all members share a launch each (160 -> 47 us
+// over three layers: 256 CTAs a launch left the last of two waves half empty).
+// Roles as in gemm_tn_persistent, with sixteen epilogue warps (a lane quadrant and
+// 32 columns each), because four members leave no room for a second accumulator
+// and the statistics are exposed: eight warps, with the results through shared
+// memory and bulk copies, took 297 us; blocks of 64 columns, two at a time, 345.
+// Every value sees ensemble_stats' operations in
 // its order.
 // ---------------------------------------------------------------------------
 struct EnsembleArgs {
-    CUtensorMap a[kMaxGroup], b[kMaxGroup], mean, spread;
+    CUtensorMap a[kMaxGroup], b[kMaxGroup];
     const float* bias[kMaxGroup];
+    float *mean, *spread;  // [rows][N], 32-byte aligned
     float scale, mid, lo, hi;
 };
-constexpr int kEBN = 128, kEStage = kUTileA + kEBN * UBK * 2, kEStages = 4;
-constexpr int kEWarps = 8;  // of the epilogue
+constexpr int kEBN = 128, kEStage = kUTileA + kEBN * UBK * 2, kEStages = 6;
+constexpr int kEWarps = 16;  // of the epilogue
 constexpr int kEThreads = 64 + 32 * kEWarps;
-constexpr size_t kESmem = (size_t)kEStages * kEStage + kEWarps * (8192 + kMaxGroup * 32 * sizeof(float)) + 1024 + 256;
+constexpr size_t kESmem = (size_t)kEStages * kEStage + kEWarps * kMaxGroup * 32 * sizeof(float) + 1024 + 256;
+
+// 8 columns of this lane's row; they are there after tcgen05.wait::ld.
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, float* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(addr));
+}
 
 template <int M>
 __global__ void __launch_bounds__(kEThreads, 1)
@@ -1260,8 +1284,7 @@ __global__ void __launch_bounds__(kEThreads, 1)
     unsigned char* base = (unsigned char*)(((uintptr_t)usmem + 1023) & ~(uintptr_t)1023);
     auto tA = [&](int st) { return base + st * kEStage; };
     auto tB = [&](int st) { return base + st * kEStage + kUTileA; };
-    unsigned char* stg_all = base + kEStages * kEStage;
-    float* sbias_all = (float*)(stg_all + kEWarps * 8192);
+    float* sbias_all = (float*)(base + kEStages * kEStage);
     uint64_t* full = (uint64_t*)(sbias_all + kEWarps * kMaxGroup * 32);
     uint64_t* empty = full + kEStages;
     uint64_t* acc_full = empty + kEStages;      // [kBufs]
@@ -1333,41 +1356,38 @@ __global__ void __launch_bounds__(kEThreads, 1)
             }
         }
     } else {
-        const int q = warp & 3, half = (warp - 2) >> 2;
-        unsigned char* stg = stg_all + (warp - 2) * 8192;  // a piece of the mean, one of the spread
+        const int q = warp & 3, c = 32 * ((warp - 2) >> 2);  // this warp's rows and columns of a block
         float* sbias = sbias_all + (warp - 2) * kMaxGroup * 32;
         const float inv = 1.f / (float)M;
-        int i = 0, n = 0;
+        int i = 0;
         for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
             const int a = i % kBufs;
-            const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * kEBN;
+            const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * kEBN + c;
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < M; ++k) sbias[k * 32 + lane] = t.bias[k][bn + lane];
+            __syncwarp();
             ok &= mbar_wait(&acc_full[a], (i / kBufs) & 1);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const size_t out = (size_t)(bm + q * 32 + lane) * N + bn;
 #pragma unroll 1
-            for (int c = 2 * half; c < 2 * half + 2; ++c, ++n) {
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < M; ++k) sbias[k * 32 + lane] = t.bias[k][bn + c * 32 + lane];
-                __syncwarp();
-                float x[M][32];
+            for (int h = 0; h < 32; h += 8) {
+                float x[M][8];
 #pragma unroll
                 for (int k = 0; k < M; ++k)
-                    tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((a * M + k) * kEBN + c * 32), x[k]);
-                if (c == 2 * half + 1) {
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0)
-                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[a])) : "memory");
-                }
-                uint32_t mean[32], spread[32];
+                    tmem_ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((a * M + k) * kEBN + c + h), x[k]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                uint32_t mean[8], spread[8];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    float s = 0.f, d = 0.f;
+                for (int j = 0; j < 8; ++j) {
+                    float s, d = 0.f;
 #pragma unroll
                     for (int k = 0; k < M; ++k) {
-                        x[k][j] = member_tl(x[k][j] + sbias[k * 32 + j], t.scale, t.mid, t.lo, t.hi);
-                        s += x[k][j];
+                        // the loads land at the wait: no use of x may move above it
+                        asm volatile("" : "+f"(x[k][j]));
+                        x[k][j] = member_tl(x[k][j] + sbias[k * 32 + h + j], t.scale, t.mid, t.lo, t.hi);
+                        s = k ? s + x[k][j] : x[k][j];
                     }
                     s *= inv;
 #pragma unroll
@@ -1375,21 +1395,16 @@ __global__ void __launch_bounds__(kEThreads, 1)
                     mean[j] = __float_as_uint(s);
                     spread[j] = __float_as_uint(sqrtf(d * inv));
                 }
-                if (n > 0) {  // the copies of the last pieces have read them
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                if (h == 24) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[a])) : "memory");
                 }
-                put_row(stg, lane, mean);
-                put_row(stg + 4096, lane, spread);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) {
-                    tma_store_2d(&t.mean, bn + c * 32, bm + q * 32, stg);
-                    tma_store_2d(&t.spread, bn + c * 32, bm + q * 32, stg + 4096);
-                }
+                store_sector(t.mean + out + h, mean);
+                store_sector(t.spread + out + h, spread);
             }
         }
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     __syncwarp();
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
@@ -1483,6 +1498,8 @@ cudaError_t launch_persistent(const TileOperands& o, const EpiArgs& e, int* err,
     f<<<std::min(blocks, sms), kPThreads, kPSmem, st>>>(t, o.M, o.N, o.K, err);
     return cudaGetLastError();
 }
+
+bool aligned32(const void* p) { return ((uintptr_t)p & 31) == 0; }
 
 // The persistent kernel once every SM has two of its blocks (256 columns; 78 us
 // at 8192 x 8192 x 512, 91 by blocks of gemm_tn_tile), else the widest block that
@@ -1779,7 +1796,7 @@ namespace {
 bool ensemble_fits(const cr_mlp_net* const* nets, int members, int batch, const void* x, int ldx, int tc,
                    const float* mean, const float* spread) {
     if (!tc || members < 2 || members > kMaxGroup || gemm_feed() != 1 || ldx < nets[0]->dims[0] || ldx % 8 ||
-        !aligned16(x) || !aligned16(mean) || !aligned16(spread))
+        !aligned16(x) || !aligned32(mean) || !aligned32(spread))
         return false;
     const int L = nets[0]->layers;
     for (int k = 0; k < members; ++k) {
@@ -1832,8 +1849,8 @@ int cr_mlp_ensemble_predict(const cr_mlp_net* const* nets, int members, int batc
             return CR_MLP_ECUDA;
         t.bias[k] = nets[k]->b[L - 1];
     }
-    if (!tile_map(&t.mean, mean, false, batch, N, N, 32) || !tile_map(&t.spread, spread, false, batch, N, N, 32))
-        return CR_MLP_ECUDA;
+    t.mean = mean;
+    t.spread = spread;
     t.scale = scale;
     t.mid = mid;
     t.lo = lo;
