@@ -1416,7 +1416,8 @@ double reg_step_us(int cluster, int rows) {
 // every ray whose column fits the registers of at most 16 CTAs.  Against the
 // batched kernel (72-78e9 term-rows per second at any depth, bound by its
 // streams from memory) it marched 123e9 on one CTA of 380 rows, 107e9 on two,
-// 104e9 at 2300 and 3800 rows and 78e9 at 5700 rows (16 CTAs of 12 rows a lane).
+// 104e9 at 2300 and 3800 rows and 82e9 at 5300 - 5700 rows (16 CTAs of 11 or 12
+// rows a lane; of 12 alone: 78e9).
 //
 // The cluster of a ray is the one that minimises the larger of its own march
 // and the whole batch's at that shape's throughput: long rays of an uneven

@@ -27,8 +27,9 @@
 //     exchange h and y of the slice to every CTA of the cluster
 //     fold     gin, xin of the slice: weighted sums over all slices' h and y
 //     sweep    true g from the lane's e, true x from its v
-//     sum      u = c_inf u + sum_k c_k x_k, two terms added in registers
-//              before the rest meet in shared memory
+//     sum      u = c_inf u + sum_k c_k x_k through shared memory; segments of
+//              ten rows and more have room for half of the terms there, and two
+//              terms are added in registers before
 //
 // Exchange.  A slice's h and y (32 bytes a term) are written straight into the
 // shared memory of every CTA (st.async), completing on a barrier of the
@@ -93,7 +94,7 @@ static_assert(sizeof(RegCtl) <= kCtlBytes, "RegCtl must fit its slot");
 // same): the CTA's own part, then one region per term, then the pairs' sums.
 // Within the first two every offset is a constant, so that a warp addresses
 // all its tables from one base.
-template <int L>
+template <int L, bool ALL>
 struct RegOff {
     static constexpr unsigned P = 32u * (unsigned)L;
     static constexpr unsigned ck = 0;                      // residues of the active set
@@ -120,11 +121,12 @@ struct RegOff {
     static constexpr unsigned wghost = xh + 32;            // -w of row R0 - 1
     static constexpr unsigned bar = wghost + 16;           // [2] mbarriers of the mailboxes
     static constexpr unsigned term = bar + 16;             // size of a region
-    // [pair][P] c_k x_k; over the same bytes, during a factorisation, the
-    // Galerkin rows [3][P]
+    // ALL: [term][P] x_k, else [pair][P] c_k x_k of two terms; over the same
+    // bytes, during a factorisation, the Galerkin rows [3][P]
     __host__ __device__ static unsigned X(int terms) { return term0 + (unsigned)terms * term; }
     __host__ __device__ static unsigned F3(int terms) {
-        return X(terms) + (unsigned)((terms + 1) / 2 > 3 ? (terms + 1) / 2 : 3) * 16 * P;
+        const int rows = ALL ? terms : (terms + 1) / 2;
+        return X(terms) + (unsigned)(rows > 3 ? rows : 3) * 16 * P;
     }
     // f3 of rows R0 - 1 .. R1 + 1, for grid outputs only
     __host__ __device__ static unsigned bytes(int terms, int nmax, int grids) {
@@ -384,10 +386,10 @@ __device__ __noinline__ void reg_weights(double2* tot, double2* WA, double2* WB,
 // Called by every thread of every CTA of the cluster (two cluster barriers
 // when C > 1).  The Galerkin rows are computed once per slice and shared by
 // its terms.
-template <int L>
+template <int L, bool ALL>
 __device__ __forceinline__ void reg_factor(const ColArgs& a, const RegCtx& x, cg::cluster_group& cl, int set,
                                            int n_active, double2 (&al)[L], double2 (&mw)[L]) {
-    using O = RegOff<L>;
+    using O = RegOff<L, ALL>;
     constexpr int P = 32 * L;
     const int k = x.term, l = x.lane;
     const bool active = k < n_active;
@@ -501,9 +503,9 @@ __device__ __noinline__ void reg_assemble(const ColArgs& a, const RegCtl* ctl, i
 }
 
 // The self-starter's delta in the slice and its halo (cupyram.py:1008-1022).
-template <int L>
+template <int L, bool ALL>
 __device__ __noinline__ void reg_source(const ColArgs& a, RegCtx x) {
-    using O = RegOff<L>;
+    using O = RegOff<L, ALL>;
     const RegCtl& s = *x.ctl;
     const RayDev ry = a.rays[s.rid];
     const EnvPtrs e = env_ptrs(a.envs[ry.env], a.pool);
@@ -585,9 +587,9 @@ __device__ __noinline__ void reg_updat(int rn, RegCtl* ctl) {
 
 // f3 of rows max(lo, R0 - 1) .. min(hi, R1 + 1) into shared memory, and the
 // weights of the line's rows with it.
-template <int L>
+template <int L, bool ALL>
 __device__ __noinline__ void reg_load_f3(const ColArgs& a, RegCtx x, int lo, int hi) {
-    float* F3 = x.at<float>(RegOff<L>::F3(blockDim.x >> 5));
+    float* F3 = x.at<float>(RegOff<L, ALL>::F3(blockDim.x >> 5));
     RegCtl* ctl = x.ctl;
     const int first = max(lo, ctl->R0 - 1), last = a.compute_grids ? min(hi, ctl->R1 + 1) : -1;
     for (int i = first + (int)threadIdx.x; i <= last; i += blockDim.x)
@@ -604,9 +606,9 @@ __device__ __noinline__ void reg_load_f3(const ColArgs& a, RegCtx x, int lo, int
 }
 
 // Offset of the field of a row in [R0 - 1, R1 + 1].
-template <int L>
+template <int L, bool ALL>
 __device__ __forceinline__ unsigned u_offset(const RegCtl& s, int row) {
-    using O = RegOff<L>;
+    using O = RegOff<L, ALL>;
     if (row < 1 || row > s.nz) return O::misc + 48;
     if (row == s.R0 - 1) return O::misc + 16;
     if (row == s.R1 + 1) return O::misc + 32;
@@ -614,26 +616,26 @@ __device__ __forceinline__ unsigned u_offset(const RegCtl& s, int row) {
 }
 
 // The outputs' part of the CTA's state (one thread).
-template <int L>
+template <int L, bool ALL>
 __device__ __noinline__ void reg_outputs(const ColArgs& a, RegCtl* ctl) {
     const RayDev& ry = a.rays[ctl->rid];
     const int ir = (int)floor(ry.zr / ry.dz), irow = max(ir, 1);
     const bool mine = irow >= ctl->R0 && irow <= ctl->R1;
     ctl->line = mine ? ry.line_off : -1;
-    ctl->ua = mine ? u_offset<L>(*ctl, ir) : 0;
-    ctl->ub = mine ? u_offset<L>(*ctl, ir + 1) : 0;
+    ctl->ua = mine ? u_offset<L, ALL>(*ctl, ir) : 0;
+    ctl->ub = mine ? u_offset<L, ALL>(*ctl, ir + 1) : 0;
     ctl->grid = a.compute_grids ? ry.grid_off : -1;
     ctl->ndz = (unsigned)ry.ndz;
     ctl->ndz_inv = ry.ndz > 1 ? (unsigned)((0x100000000ull + ry.ndz - 1) / (unsigned)ry.ndz) : 0u;
     ctl->nvz = ry.nvz;
 }
 
-// The sum over N pairs of terms of the rows j = k, k + terms, .. of this lane
-// (and outputs among them).
-template <int L, int N>
+// The sum over N terms (ALL) or pairs of terms of the rows j = k, k + terms, ..
+// of this lane (and outputs among them).
+template <int L, bool ALL, int N>
 __device__ __forceinline__ void reg_sum(const ColArgs& a, const RegCtx& x, double2 ci, int k, int l, int terms,
                                         int out) {
-    using O = RegOff<L>;
+    using O = RegOff<L, ALL>;
     constexpr unsigned P16 = 512u * L;
     const unsigned us = x.sm32 + O::U + 16u * (unsigned)l, xs0 = x.sm32 + O::X(terms) + 16u * (unsigned)l;
 #pragma unroll 1
@@ -643,8 +645,19 @@ __device__ __forceinline__ void reg_sum(const ColArgs& a, const RegCtx& x, doubl
 #pragma unroll
         for (int q = 0; q < N; ++q) xs[q] = lds2(xa + (unsigned)q * P16);
         double2 acc = cmul(ci, lds2(ua));
+        if (ALL) {  // two chains of c_k x_k
+            double2 other = c2(0.0, 0.0);
 #pragma unroll
-        for (int q = 0; q < N; ++q) acc = cadd(acc, xs[q]);
+            for (int q = 0; q < N; ++q) {
+                const double2 ck = lds2(x.sm32 + O::ck + 16u * (unsigned)q);
+                if (q & 1) other = vfma(ck, xs[q], other);
+                else acc = vfma(ck, xs[q], acc);
+            }
+            acc = cadd(acc, other);
+        } else {
+#pragma unroll
+            for (int q = 0; q < N; ++q) acc = cadd(acc, xs[q]);
+        }
         // positions without a row stay zero
         if (j >= x.npad) sts2(ua, acc);
         if (out >= 0 && x.ctl->grid >= 0 && j >= x.npad) {
@@ -664,10 +677,10 @@ __device__ __forceinline__ void reg_sum(const ColArgs& a, const RegCtx& x, doubl
 // One range step of the active set; out >= 0: the step's field is output
 // `out` (outpt.py:11-57; transmission loss follows at the end, reg_tl).
 // step: index of the step, the self-starter's three included.
-template <int L>
+template <int L, bool ALL>
 __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int na, const double2 (&al)[L],
                                          const double2 (&mw)[L], int step, int out) {
-    using O = RegOff<L>;
+    using O = RegOff<L, ALL>;
     constexpr unsigned P16 = 512u * L;  // bytes of a per-row table
     const int k = x.term, l = x.lane, terms = (int)(blockDim.x >> 5);
     const unsigned sm = x.sm32, tm = x.tm32, us = sm + O::U + 16u * (unsigned)l;
@@ -796,11 +809,15 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
             sts2(tm + O::xh, cmul(ck, vfma(lds2(tm + O::wghost), v, lds2(tm + O::xh))));
             sts2(tm + O::xh + 16u, cmul(ck, lds2(tm + O::xh + 16u)));
         }
-        // the terms' share of the sum.  Warps k and k + half are a pair: each leaves
-        // the other's half of the rows and adds its own half to what the other left.
-        const bool up_warp = k >= half;
+        // the terms' share of the sum
+        const bool up_warp = !ALL && k >= half;
         const unsigned xa = sm + O::X(terms) + 16u * (unsigned)l + (unsigned)(up_warp ? k - half : k) * P16;
-        if (up_warp || k + half < na) {
+        if (ALL) {
+#pragma unroll
+            for (int j = 0; j < L; ++j) sts2(xa + j * 512u, g[j]);
+        } else if (up_warp || k + half < na) {
+            // warps k and k + half are a pair: each leaves the other's half of the rows
+            // and adds its own half to what the other left
             constexpr int H = L / 2;
             if (up_warp) {
 #pragma unroll
@@ -821,14 +838,29 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
         }
     }
     __syncthreads();
-    // u = c_inf u + the pairs' sums
+    // u = c_inf u + the terms' or pairs' sums
     const double2 ci = lds2(sm + O::misc);
-    switch (half) {
-        case 1: reg_sum<L, 1>(a, x, ci, k, l, terms, out); break;
-        case 2: reg_sum<L, 2>(a, x, ci, k, l, terms, out); break;
-        case 3: reg_sum<L, 3>(a, x, ci, k, l, terms, out); break;
-        case 4: reg_sum<L, 4>(a, x, ci, k, l, terms, out); break;
-        default: reg_sum<L, 5>(a, x, ci, k, l, terms, out); break;
+    if constexpr (ALL) {
+        switch (na) {
+            case 1: reg_sum<L, ALL, 1>(a, x, ci, k, l, terms, out); break;
+            case 2: reg_sum<L, ALL, 2>(a, x, ci, k, l, terms, out); break;
+            case 3: reg_sum<L, ALL, 3>(a, x, ci, k, l, terms, out); break;
+            case 4: reg_sum<L, ALL, 4>(a, x, ci, k, l, terms, out); break;
+            case 5: reg_sum<L, ALL, 5>(a, x, ci, k, l, terms, out); break;
+            case 6: reg_sum<L, ALL, 6>(a, x, ci, k, l, terms, out); break;
+            case 7: reg_sum<L, ALL, 7>(a, x, ci, k, l, terms, out); break;
+            case 8: reg_sum<L, ALL, 8>(a, x, ci, k, l, terms, out); break;
+            case 9: reg_sum<L, ALL, 9>(a, x, ci, k, l, terms, out); break;
+            default: reg_sum<L, ALL, 10>(a, x, ci, k, l, terms, out); break;
+        }
+    } else {
+        switch (half) {
+            case 1: reg_sum<L, ALL, 1>(a, x, ci, k, l, terms, out); break;
+            case 2: reg_sum<L, ALL, 2>(a, x, ci, k, l, terms, out); break;
+            case 3: reg_sum<L, ALL, 3>(a, x, ci, k, l, terms, out); break;
+            case 4: reg_sum<L, ALL, 4>(a, x, ci, k, l, terms, out); break;
+            default: reg_sum<L, ALL, 5>(a, x, ci, k, l, terms, out); break;
+        }
     }
     if (k == terms - 1) {
         // halo rows outside the column (rows 0 and nz + 1) stay zero: lane 2 t + h
@@ -887,10 +919,10 @@ __device__ __noinline__ void reg_tl(const ColArgs& a, int rid, int C, int c, int
 template <int L>
 constexpr int reg_cap() { return L >= 8 ? 168 : 128; }
 
-template <int L>
+template <int L, bool ALL>
 __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant__ ColArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    using O = RegOff<L>;
+    using O = RegOff<L, ALL>;
     cg::cluster_group cl = cg::this_cluster();
     RegCtx x;
     x.sm = smem_raw;
@@ -945,11 +977,11 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
     __syncthreads();
     reg_assemble(a, ctl, 0, ctl->nz + 1);
     if (threadIdx.x == 0) {
-        reg_source<L>(a, x);
-        reg_outputs<L>(a, ctl);
+        reg_source<L, ALL>(a, x);
+        reg_outputs<L, ALL>(a, ctl);
     }
     cl.sync();  // every CTA's mailboxes are ready
-    reg_load_f3<L>(a, x, 0, ctl->nz + 1);
+    reg_load_f3<L, ALL>(a, x, 0, ctl->nz + 1);
     const int n = ctl->n;
     {
         int start, cnt;
@@ -987,7 +1019,7 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
             refactor = ctl->refactor;
             if (ctl->lo <= ctl->hi) {
                 reg_assemble(a, ctl, ctl->lo, ctl->hi);
-                reg_load_f3<L>(a, x, ctl->lo, ctl->hi);
+                reg_load_f3<L, ALL>(a, x, ctl->lo, ctl->hi);
             }
         }
         if (refactor) {
@@ -999,7 +1031,7 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
                         (int)threadIdx.x < na ? a.pfc[base + threadIdx.x] : c2(0.0, 0.0);
                 if (threadIdx.x == 0) misc[0] = a.pfcinf[(long long)ctl->rid * kSets + want];
             }
-            reg_factor<L>(a, x, cl, want, na, al, mw);
+            reg_factor<L, ALL>(a, x, cl, want, na, al, mw);
             if (threadIdx.x == 0) ctl->set = want;
         }
         // the steps that this operator serves
@@ -1011,7 +1043,7 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
                 if (tlc < ctl->nvr) out = tlc;
                 ++tlc;
             }
-            reg_step<L>(a, x, na, al, mw, q, out);
+            reg_step<L, ALL>(a, x, na, al, mw, q, out);
         }
     }
     if (threadIdx.x == 0 && ctl->dead) atomicOr(a.flags + ctl->rid, 2);
@@ -1020,28 +1052,54 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
     reg_tl(a, ctl->rid, x.C, x.c, min(tlc, ctl->nvr));
 }
 
-constexpr int kRows[] = {1, 2, 3, 4, 5, 6, 8, 10, 12};
+constexpr int kRows[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12};
+
+// Longest segment whose terms may each leave their solution to the sum (see
+// reg_kernel): longer ones need the room.
+constexpr int kAllRows = 9;
 
 // The kernel of L rows a lane and its shared memory.
 struct RegKernel {
     const void* f = nullptr;
     unsigned (*bytes)(int terms, int nmax, int grids) = nullptr;
+    int regs = 0;
 };
+template <int L, bool ALL>
+RegKernel reg_kernel_of() { return {(const void*)march_reg_kernel<L, ALL>, RegOff<L, ALL>::bytes, reg_cap<L>()}; }
 template <int L>
-RegKernel reg_kernel_of() { return {(const void*)march_reg_kernel<L>, RegOff<L>::bytes}; }
-RegKernel reg_kernel(int L) {
+RegKernel reg_kernel_at(bool all) {
+    if constexpr (L <= kAllRows)
+        if (all) return reg_kernel_of<L, true>();
+    return reg_kernel_of<L, false>();
+}
+RegKernel reg_kernel(int L, bool all) {
     switch (L) {
-        case 1: return reg_kernel_of<1>();
-        case 2: return reg_kernel_of<2>();
-        case 3: return reg_kernel_of<3>();
-        case 4: return reg_kernel_of<4>();
-        case 5: return reg_kernel_of<5>();
-        case 6: return reg_kernel_of<6>();
-        case 8: return reg_kernel_of<8>();
-        case 10: return reg_kernel_of<10>();
-        case 12: return reg_kernel_of<12>();
+        case 1: return reg_kernel_at<1>(all);
+        case 2: return reg_kernel_at<2>(all);
+        case 3: return reg_kernel_at<3>(all);
+        case 4: return reg_kernel_at<4>(all);
+        case 5: return reg_kernel_at<5>(all);
+        case 6: return reg_kernel_at<6>(all);
+        case 7: return reg_kernel_at<7>(all);
+        case 8: return reg_kernel_at<8>(all);
+        case 9: return reg_kernel_at<9>(all);
+        case 10: return reg_kernel_at<10>(all);
+        case 11: return reg_kernel_at<11>(all);
+        case 12: return reg_kernel_at<12>(all);
     }
     return {};
+}
+// Every term leaves its x to the sum - no pairs that wait for one another - where
+// that takes no CTA off an SM.  256 wedge rays 42.8 -> 40.2 ms, 30 of them 18.3 ->
+// 15.7; single rays of 16 CTAs stay (12.5 and 12.6 ms).
+RegKernel reg_kernel(int L, int terms, int nmax, int grids) {
+    const RegKernel pairs = reg_kernel(L, false), all = reg_kernel(L, true);
+    if (!pairs.f || all.f == pairs.f) return pairs;
+    const int by_regs = 65536 / (pairs.regs * 32 * terms);
+    auto ctas = [&](const RegKernel& kn) {
+        return std::min(by_regs, (int)(228 * 1024 / (kn.bytes(terms, nmax, grids) + 1024)));
+    };
+    return all.bytes(terms, nmax, grids) <= kRegSmemLimit && ctas(all) >= ctas(pairs) ? all : pairs;
 }
 
 cudaError_t reg_config(const RegKernel& kn, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int n_rays, int cluster,
@@ -1068,7 +1126,7 @@ cudaError_t reg_config(const RegKernel& kn, cudaLaunchConfig_t& cfg, cudaLaunchA
 }
 
 bool reg_shape_ok(int cluster, int terms, int rows) {
-    return terms >= 1 && terms <= kRegMaxTerms && cluster >= 1 && cluster <= kRegMaxCluster && reg_kernel(rows).f;
+    return terms >= 1 && terms <= kRegMaxTerms && cluster >= 1 && cluster <= kRegMaxCluster && reg_kernel(rows, false).f;
 }
 
 }  // namespace
@@ -1084,7 +1142,7 @@ int reg_rows(int nz, int cluster) {
 cudaError_t launch_march_reg(const ColArgs& a, int n_rays, int cluster, int terms, int rows, int nz_max,
                              cudaStream_t st) {
     if (!reg_shape_ok(cluster, terms, rows)) return cudaErrorInvalidValue;
-    const RegKernel kn = reg_kernel(rows);
+    const RegKernel kn = reg_kernel(rows, terms, (nz_max + cluster - 1) / cluster, a.compute_grids);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     cudaError_t ce = reg_config(kn, cfg, attr, n_rays, cluster, terms, nz_max, a.compute_grids, st);
@@ -1096,7 +1154,7 @@ cudaError_t launch_march_reg(const ColArgs& a, int n_rays, int cluster, int term
 
 int reg_max_active_clusters(int cluster, int terms, int rows, int nz_max, int grids) {
     if (!reg_shape_ok(cluster, terms, rows)) return 0;
-    const RegKernel kn = reg_kernel(rows);
+    const RegKernel kn = reg_kernel(rows, terms, (nz_max + cluster - 1) / cluster, grids);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     if (reg_config(kn, cfg, attr, 1, cluster, terms, nz_max, grids, 0) != cudaSuccess) return 0;

@@ -92,3 +92,15 @@ def test_changed_order_of_a_set(cuda_device):
         a, c = eng.run(), ref.run()
     n = b.line_len
     assert np.abs(a["cpl"][:n] - c["cpl"][:n]).max() < 1e-6 * np.abs(c["cpl"][:n]).max()
+
+
+# segments of 7, 9 and 11 rows at their edges; the sum over all terms or over pairs (8 and 10 terms leave less room)
+@pytest.mark.parametrize("nz,npd", [(193, 1), (224, 6), (193, 8), (224, 10), (257, 3), (288, 6), (288, 7), (321, 2),
+                                    (352, 6), (352, 8), (160, 8), (160, 10), (320, 6)])
+def test_odd_segments_and_sums_vs_oracle(cuda_device, nz, npd):
+    rays = 300
+    b = _batch(nz, npd, rays, True)
+    with Engine(b) as eng:
+        out = eng.run()
+        assert eng.stats()["rays_failed"] == 0 and eng.stats()["n_tiles"] == 0
+    _check(_batch(nz, npd, 1, True), {k: out[k] for k in ("tll", "cpl")}, out["cpg"])
