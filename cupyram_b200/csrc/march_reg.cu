@@ -27,9 +27,8 @@
 //     exchange h and y of the slice to every CTA of the cluster
 //     fold     gin, xin of the slice: weighted sums over all slices' h and y
 //     sweep    true g from the lane's e, true x from its v
-//     sum      u = c_inf u + sum_k c_k x_k through shared memory; segments of
-//              ten rows and more have room for half of the terms there, and two
-//              terms are added in registers before
+//     sum      u = c_inf u + sum_k c_k x_k, two terms added in registers
+//              before the rest meet in shared memory
 //
 // Exchange.  A slice's h and y (32 bytes a term) are written straight into the
 // shared memory of every CTA (st.async), completing on a barrier of the
@@ -660,7 +659,7 @@ __device__ __forceinline__ void reg_sum(const ColArgs& a, const RegCtx& x, doubl
         }
         // positions without a row stay zero
         if (j >= x.npad) sts2(ua, acc);
-        if (out >= 0 && x.ctl->grid >= 0 && j >= x.npad) {
+        if (a.compute_grids && out >= 0 && x.ctl->grid >= 0 && j >= x.npad) {
             const RegCtl* ctl = x.ctl;
             int start, cnt;
             lane_rows(ctl->n, l, start, cnt);
@@ -774,13 +773,10 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
                 ev = lds2(tl + O::EV);
             }
             double2 f = vfma(wb, my, cmul(wa, mh));
-            if (x.C > 4) {
-                f = cadd(f, shfl2_xor(f, 8));
-                f = cadd(f, shfl2_xor(f, 4));
-            }
-            f = cadd(f, shfl2_xor(f, 2));
-            f = cadd(f, shfl2_xor(f, 1));
-            const double2 gin = shfl2(f, 0), xin = shfl2(f, 16);
+#pragma unroll
+            for (int d = 8; d >= 1; d >>= 1) f = cadd(f, shfl2_xor(f, d));
+            const double2 other = shfl2_xor(f, 16);
+            const double2 gin = l < 16 ? f : other, xin = l < 16 ? other : f;
             // for the halo rows, once the lane's x are known
             if (l == 0) sts2(tm + O::xh, gin);
             if (l == 0) sts2(tm + O::xh + 16u, xin);
@@ -875,7 +871,7 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
             const bool inside = l == 0 ? ctl->R0 > 1 : ctl->R1 < ctl->nz;
             acc = vfma(ci, old, acc);
             sts2(sm + O::misc + 16u + 16u * hh, inside ? acc : c2(0.0, 0.0));
-            if (out >= 0 && l == 1 && !inside && ctl->grid >= 0) {  // grid row nz + 1: zero
+            if (a.compute_grids && out >= 0 && l == 1 && !inside && ctl->grid >= 0) {  // grid row nz + 1: zero
                 const unsigned row = (unsigned)ctl->nz + 1u, q = row / ctl->ndz;
                 if (q * ctl->ndz == row && (int)q <= ctl->nvz)
                     a.cpg[ctl->grid + (long long)(q - 1) * ctl->nvr + out] = c2(0.0, 0.0);
@@ -1090,8 +1086,7 @@ RegKernel reg_kernel(int L, bool all) {
     return {};
 }
 // Every term leaves its x to the sum - no pairs that wait for one another - where
-// that takes no CTA off an SM.  256 wedge rays 42.8 -> 40.2 ms, 30 of them 18.3 ->
-// 15.7; single rays of 16 CTAs stay (12.5 and 12.6 ms).
+// that takes no CTA off an SM.
 RegKernel reg_kernel(int L, int terms, int nmax, int grids) {
     const RegKernel pairs = reg_kernel(L, false), all = reg_kernel(L, true);
     if (!pairs.f || all.f == pairs.f) return pairs;
