@@ -85,8 +85,12 @@ struct RegCtl {
     int env, n_bt, n_rss, n_rsb;
     double dr, dz;
     const double *rb, *zb, *rp_ss, *rp_sb;
+    double inv_dr, inv_per;  // 1 / dr; steps a cell of the bottom's segment takes (segment per_bt)
+    int per_bt;
+    int line_row;            // the line lies between this row and the next,
+    double line_dir;         // this far down
 };
-constexpr unsigned kCtlBytes = 256;
+constexpr unsigned kCtlBytes = 320;
 static_assert(sizeof(RegCtl) <= kCtlBytes, "RegCtl must fit its slot");
 
 // Shared memory of a CTA (offsets in bytes; every CTA of a cluster uses the
@@ -348,8 +352,8 @@ __device__ __noinline__ void reg_weights(double2* tot, double2* WA, double2* WB,
     // lane i: the products of A over i .. c - 1 and of Z over c + 1 .. i, and then
     // without the first and the last
     double2 pa = i < c ? A : one, pz = i > c ? Z : one;
-#pragma unroll
-    for (int d = 1; d < 16; d <<= 1) {
+#pragma unroll 1
+    for (int d = 1; d < C; d <<= 1) {
         const double2 qa = shfl2(pa, min(i + d, 31)), qz = shfl2(pz, max(i - d, 0));
         pa = i + d < 32 ? cmul(pa, qa) : pa;
         pz = i >= d ? cmul(pz, qz) : pz;
@@ -364,8 +368,8 @@ __device__ __noinline__ void reg_weights(double2* tot, double2* WA, double2* WB,
         T = zero;
         M = one;
     }
-#pragma unroll
-    for (int d = 1; d < 16; d <<= 1) {
+#pragma unroll 1
+    for (int d = 1; d < C; d <<= 1) {
         const double2 qm = shfl2(M, min(i + d, 31)), qt = shfl2(T, min(i + d, 31));
         if (i + d < 32) {
             T = vfma(M, qt, T);
@@ -533,14 +537,17 @@ __device__ __noinline__ void reg_source(const ColArgs& a, RegCtx x) {
 // first step that has to be looked at again.  Steps in between cannot change
 // the operator: the next profile, bottom segment or stability range lies
 // further on, and the bottom's depth index (linear in range within a segment)
-// stays in its cell; both bounds keep a step's margin for rounding.
+// stays in its cell; both bounds keep a step's margin for rounding.  One thread's
+// seven divisions were 1.6 us of a step whose operator changes: the bounds multiply
+// by reciprocals kept for the march and for the bottom's segment; the depth index
+// itself is divided as the reference divides it.
 __device__ __noinline__ void reg_updat(int rn, RegCtl* ctl) {
     const RegCtl& e = *ctl;
     const double dr = e.dr, r = (double)(rn + 1) * dr;
     bool reprofile = false;
     int iz = ctl->iz, ss = ctl->ss, sb = ctl->sb, bt = ctl->bt, set = ctl->set == 1 ? 2 : ctl->set;
     double stay = 1e9;  // steps that cannot change anything
-    auto event = [&](double v) { stay = fmin(stay, floor(v / dr) - 2.0 - (double)rn); };
+    auto event = [&](double v) { stay = fmin(stay, floor(v * e.inv_dr) - 2.0 - (double)rn); };
     if (e.n_bt > 1) {
         while (bt < e.n_bt - 1 && r >= e.rb[bt + 1]) ++bt;
         const int b1 = min(bt + 1, e.n_bt - 1);
@@ -549,9 +556,12 @@ __device__ __noinline__ void reg_updat(int rn, RegCtl* ctl) {
         iz = max(1, min(e.nz - 1, (int)floor(zc / e.dz)));
         if (b1 != bt) {
             event(r1);
-            const double f = zc / e.dz, per = (z1 - z0) / (r1 - r0) * dr / e.dz;
-            if (per > 0.0) stay = fmin(stay, floor((floor(f) + 1.0 - f) / per) - 1.0);
-            if (per < 0.0) stay = fmin(stay, floor((floor(f) - f) / per) - 1.0);
+            if (bt != e.per_bt) {
+                ctl->per_bt = bt;
+                ctl->inv_per = e.dz * (r1 - r0) / ((z1 - z0) * dr);  // infinite where the bottom is flat
+            }
+            const double f = zc / e.dz, inv_per = e.inv_per;
+            if (z1 != z0) stay = fmin(stay, floor((inv_per > 0.0 ? floor(f) + 1.0 - f : floor(f) - f) * inv_per) - 1.0);
         }
     }
     if (e.n_rss > 1) {
@@ -594,11 +604,8 @@ __device__ __noinline__ void reg_load_f3(const ColArgs& a, RegCtx x, int lo, int
     for (int i = first + (int)threadIdx.x; i <= last; i += blockDim.x)
         F3[i - (ctl->R0 - 1)] = a.f3[ctl->col + (long long)i * kTile];
     if (threadIdx.x == 0 && ctl->line >= 0) {
-        const RayDev& ry = a.rays[ctl->rid];
-        const double ri = ry.zr / ry.dz;
-        const int ir = (int)floor(ri);
-        const double dir = ri - ir;
-        const long long o = ctl->col + (long long)ir * kTile;
+        const double dir = ctl->line_dir;
+        const long long o = ctl->col + (long long)ctl->line_row * kTile;
         ctl->wa = (1.0 - dir) * (double)a.f3[o];
         ctl->wb = dir * (double)a.f3[o + kTile];
     }
@@ -621,6 +628,8 @@ __device__ __noinline__ void reg_outputs(const ColArgs& a, RegCtl* ctl) {
     const int ir = (int)floor(ry.zr / ry.dz), irow = max(ir, 1);
     const bool mine = irow >= ctl->R0 && irow <= ctl->R1;
     ctl->line = mine ? ry.line_off : -1;
+    ctl->line_row = ir;
+    ctl->line_dir = ry.zr / ry.dz - ir;
     ctl->ua = mine ? u_offset<L, ALL>(*ctl, ir) : 0;
     ctl->ub = mine ? u_offset<L, ALL>(*ctl, ir + 1) : 0;
     ctl->grid = a.compute_grids ? ry.grid_off : -1;
@@ -956,6 +965,8 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
         ctl->env = ry.env;
         ctl->dr = ry.dr;
         ctl->dz = ry.dz;
+        ctl->inv_dr = 1.0 / ry.dr;
+        ctl->per_bt = -1;
         ctl->n_bt = e.n_bt;
         ctl->n_rss = e.n_rss;
         ctl->n_rsb = e.n_rsb;
