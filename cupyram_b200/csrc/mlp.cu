@@ -566,11 +566,28 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, float* v) {
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(u[j]);
 }
 
+// Roles run by whole warps, with one elected lane at the instructions that one
+// thread issues: a loop that only lane 0 entered kept addresses and descriptors in
+// per-thread registers, and moving them over for every MMA and copy took longer than
+// a narrow MMA itself (512 x 512 x 8192 with mask 44 -> 28 us, ensemble_tile 264 ->
+// 207, 512 x 512 x 512 7.3 -> 6.4).
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// The whole warp waits, and goes on or gives up together.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, unsigned parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+}
+
 // The MMAs of one stage (128 rows x 64 of A, the idesc's columns x 64 of B), by one thread.
 __device__ __forceinline__ void mma_stage(uint32_t acc, uint32_t sa, uint32_t sb, uint32_t idesc, bool first) {
+    const uint64_t da0 = umma_desc_sw128(sa), db0 = umma_desc_sw128(sb);
 #pragma unroll
     for (int k = 0; k < UBK / 16; ++k) {
-        const uint64_t da = umma_desc_sw128(sa + k * 32), db = umma_desc_sw128(sb + k * 32);
+        const uint64_t da = da0 + 2 * k, db = db0 + 2 * k;  // 32 bytes on, in units of 16
         const uint32_t accum = (!first || k > 0) ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -676,7 +693,7 @@ __global__ void __launch_bounds__(kUThreads) gemm_tn_tile(const __grid_constant_
     uint64_t* done = empty + ST;
     uint64_t* mask_bar = done + 1;
     uint32_t* taddr_s = (uint32_t*)(mask_bar + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int bm = blockIdx.y * UBM, bn = blockIdx.x * BN;
 
     if (warp == 0) {
@@ -703,31 +720,39 @@ __global__ void __launch_bounds__(kUThreads) gemm_tn_tile(const __grid_constant_
     bool ok = true;
 
     int issued = 0;  // producer: tiles whose loads were issued
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         for (int kt = 0; kt < nk && ok; ++kt) {
             const int st = kt % ST;
-            if (kt >= ST) ok &= mbar_wait(&empty[st], ((kt / ST) - 1) & 1);
+            if (kt >= ST) ok = warp_wait(&empty[st], ((kt / ST) - 1) & 1);
             if (!ok) break;
-            mbar_expect_tx(&full[st], (unsigned)T::kStage);
-            tma_load_2d(tA(st), &mapA, kt * UBK, bm, &full[st]);
-            tma_load_2d(tB(st), &mapB, kt * UBK, bn, &full[st]);
-            issued = kt + 1;
-            if (kMasked && kt == 0) {
-                mbar_expect_tx(mask_bar, (unsigned)T::kMask);
+            if (elect_lane()) {
+                mbar_expect_tx(&full[st], (unsigned)T::kStage);
+                tma_load_2d(tA(st), &mapA, kt * UBK, bm, &full[st]);
+                tma_load_2d(tB(st), &mapB, kt * UBK, bn, &full[st]);
+                if (kMasked && kt == 0) {
+                    mbar_expect_tx(mask_bar, (unsigned)T::kMask);
 #pragma unroll 1
-                for (int c = 0; c < BN / 64; ++c) tma_load_2d(masks + c * UBM * 128, &mapM, bn + 64 * c, bm, mask_bar);
+                    for (int c = 0; c < BN / 64; ++c)
+                        tma_load_2d(masks + c * UBM * 128, &mapM, bn + 64 * c, bm, mask_bar);
+                }
             }
+            __syncwarp();
+            issued = kt + 1;
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         for (int kt = 0; kt < nk && ok; ++kt) {
             const int st = kt % ST;
-            ok &= mbar_wait(&full[st], (kt / ST) & 1);
+            ok = warp_wait(&full[st], (kt / ST) & 1);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            mma_stage(tmem, smem_u32(tA(st)), smem_u32(tB(st)), idesc, kt == 0);
-            mma_commit(&empty[st]);
+            if (elect_lane()) {
+                mma_stage(tmem, smem_u32(tA(st)), smem_u32(tB(st)), idesc, kt == 0);
+                mma_commit(&empty[st]);
+            }
+            __syncwarp();
         }
-        mma_commit(done);  // the accumulator is complete
+        // the accumulator is complete once every MMA issued so far is
+        if (elect_lane()) mma_commit(done);
     }
     __syncwarp();
     ok &= mbar_wait(done, 0);
@@ -1114,7 +1139,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
     uint64_t* acc_full = empty + kPStages;   // [2]
     uint64_t* acc_empty = acc_full + 2;      // [2]
     uint32_t* taddr_s = (uint32_t*)(acc_empty + 2);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int nk = K / UBK, nbm = M / UBM, nbn = N / UBN, nblocks = nbm * nbn;
 
     if (warp == 0) {
@@ -1141,42 +1166,45 @@ __global__ void __launch_bounds__(kPThreads, 1)
     int issued = 0;  // producer: k-tiles whose loads were issued (over all blocks)
 
     if (warp == 0) {
-        if (lane == 0) {
-            int g = 0;
-            for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x) {
-                const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * UBN;
-                for (int kt = 0; kt < nk && ok; ++kt, ++g) {
-                    const int st = g % kPStages;
-                    if (g >= kPStages) ok &= mbar_wait(&empty[st], ((g / kPStages) - 1) & 1);
-                    if (!ok) break;
+        int g = 0;
+        for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x) {
+            const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * UBN;
+            for (int kt = 0; kt < nk && ok; ++kt, ++g) {
+                const int st = g % kPStages;
+                if (g >= kPStages) ok = warp_wait(&empty[st], ((g / kPStages) - 1) & 1);
+                if (!ok) break;
+                if (elect_lane()) {
                     mbar_expect_tx(&full[st], (unsigned)kUStage);
                     tma_load_2d(tA(st), &t.a[0], kt * UBK, bm, &full[st]);
                     tma_load_2d(tB(st), &t.b[0], kt * UBK, bn, &full[st]);
-                    issued = g + 1;
                 }
+                __syncwarp();
+                issued = g + 1;
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            int g = 0, i = 0;
-            for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
-                const int a = i & 1;
-                // the epilogue has drained this accumulator's previous block
-                if (i >= 2) ok &= mbar_wait(&acc_empty[a], ((i / 2) - 1) & 1);
+        int g = 0, i = 0;
+        for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
+            const int a = i & 1;
+            // the epilogue has drained this accumulator's previous block
+            if (i >= 2) ok = warp_wait(&acc_empty[a], ((i / 2) - 1) & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc_addr = tmem + (uint32_t)(a * UBN);
+            for (int kt = 0; kt < nk && ok; ++kt, ++g) {
+                const int st = g % kPStages;
+                ok = warp_wait(&full[st], (g / kPStages) & 1);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc_addr = tmem + (uint32_t)(a * UBN);
-                for (int kt = 0; kt < nk && ok; ++kt, ++g) {
-                    const int st = g % kPStages;
-                    ok &= mbar_wait(&full[st], (g / kPStages) & 1);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_lane()) {
                     mma_stage(acc_addr, smem_u32(tA(st)), smem_u32(tB(st)), kUIdesc, kt == 0);
                     mma_commit(&empty[st]);
                 }
-                if (!ok) break;
-                mma_commit(&acc_full[a]);
+                __syncwarp();
             }
+            if (!ok) break;
+            if (elect_lane()) mma_commit(&acc_full[a]);
+            __syncwarp();
         }
     } else {
         // epilogue: TMEM lane quadrant q = warp mod 4 holds rows 32q..32q+31
@@ -1245,13 +1273,12 @@ __global__ void __launch_bounds__(kPThreads, 1)
 // same 128 x 128 block of every member side by side in tensor memory (M x 128
 // of the 512 columns; two members leave room for two blocks), and the epilogue
 // turns them into mean and spread in registers: only the results leave, by whole
-// 32-byte sectors of a lane's row (343 -> 264 us; the contractions' part alone is
-// 190), and the hidden layers of all members share a launch each (160 -> 47 us
+// 32-byte sectors of a lane's row (343 -> 207 us), and the hidden layers of all members share a launch each (160 -> 47 us
 // over three layers: 256 CTAs a launch left the last of two waves half empty).
 // Roles as in gemm_tn_persistent, with sixteen epilogue warps (a lane quadrant and
 // 32 columns each), because four members leave no room for a second accumulator
 // and the statistics are exposed: eight warps, with the results through shared
-// memory and bulk copies, took 297 us; blocks of 64 columns, two at a time, 345.
+// memory and bulk copies, took 33 us more; blocks of 64 columns, two at a time, 4.
 // Every value sees ensemble_stats' operations in
 // its order.
 // ---------------------------------------------------------------------------
@@ -1290,7 +1317,7 @@ __global__ void __launch_bounds__(kEThreads, 1)
     uint64_t* acc_full = empty + kEStages;      // [kBufs]
     uint64_t* acc_empty = acc_full + kBufs;     // [kBufs]
     uint32_t* taddr_s = (uint32_t*)(acc_empty + kBufs);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int nk = K / UBK, nbm = rows / UBM, nblocks = nbm * (N / kEBN);
 
     if (warp == 0) {
@@ -1317,43 +1344,46 @@ __global__ void __launch_bounds__(kEThreads, 1)
     int issued = 0;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int g = 0;
-            for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x) {
-                const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * kEBN;
-                for (int k = 0; k < M && ok; ++k)
-                    for (int kt = 0; kt < nk && ok; ++kt, ++g) {
-                        const int st = g % kEStages;
-                        if (g >= kEStages) ok &= mbar_wait(&empty[st], ((g / kEStages) - 1) & 1);
-                        if (!ok) break;
+        int g = 0;
+        for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x) {
+            const int bm = (blk % nbm) * UBM, bn = (blk / nbm) * kEBN;
+            for (int k = 0; k < M && ok; ++k)
+                for (int kt = 0; kt < nk && ok; ++kt, ++g) {
+                    const int st = g % kEStages;
+                    if (g >= kEStages) ok = warp_wait(&empty[st], ((g / kEStages) - 1) & 1);
+                    if (!ok) break;
+                    if (elect_lane()) {
                         mbar_expect_tx(&full[st], (unsigned)kEStage);
                         tma_load_2d(tA(st), &t.a[k], kt * UBK, bm, &full[st]);
                         tma_load_2d(tB(st), &t.b[k], kt * UBK, bn, &full[st]);
-                        issued = g + 1;
                     }
-            }
+                    __syncwarp();
+                    issued = g + 1;
+                }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            int g = 0, i = 0;
-            for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
-                const int a = i % kBufs;
-                if (i >= kBufs) ok &= mbar_wait(&acc_empty[a], ((i / kBufs) - 1) & 1);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int k = 0; k < M && ok; ++k)
-                    for (int kt = 0; kt < nk && ok; ++kt, ++g) {
-                        const int st = g % kEStages;
-                        ok &= mbar_wait(&full[st], (g / kEStages) & 1);
-                        if (!ok) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        int g = 0, i = 0;
+        for (int blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x, ++i) {
+            const int a = i % kBufs;
+            if (i >= kBufs) ok = warp_wait(&acc_empty[a], ((i / kBufs) - 1) & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int k = 0; k < M && ok; ++k)
+                for (int kt = 0; kt < nk && ok; ++kt, ++g) {
+                    const int st = g % kEStages;
+                    ok = warp_wait(&full[st], (g / kEStages) & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (elect_lane()) {
                         mma_stage(tmem + (uint32_t)((a * M + k) * kEBN), smem_u32(tA(st)), smem_u32(tB(st)), idesc,
                                   kt == 0);
                         mma_commit(&empty[st]);
                     }
-                if (!ok) break;
-                mma_commit(&acc_full[a]);
-            }
+                    __syncwarp();
+                }
+            if (!ok) break;
+            if (elect_lane()) mma_commit(&acc_full[a]);
+            __syncwarp();
         }
     } else {
         const int q = warp & 3, c = 32 * ((warp - 2) >> 2);  // this warp's rows and columns of a block
