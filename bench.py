@@ -228,8 +228,11 @@ def measured_peak_hbm():
     return 6650.0, "fallback"
 
 
-def profiled_traffic(form):
-    """DRAM bytes per grid-point update of the march kernel from the committed ncu summary."""
+def profiled_traffic(form, n_tiles):
+    """DRAM bytes per grid-point update of the batched march from the committed ncu summary
+    (None when no ray marches there: the register march keeps its column on the chip)."""
+    if not n_tiles:
+        return None
     p = ROOT / "profiles" / "march_traffic.json"
     if not p.exists():
         return None
@@ -304,13 +307,14 @@ def chosen_form(a, batch, out_plain, torch, world, pg, barrier, peak, form="chos
         gmax, grms = tl_errors(refs["tlg"], out["tlg"].numpy())
         errs.update(tl_grid_err_max_db=gmax, tl_grid_err_rms_db=grms,
                     tl_grid_cells=int(np.sum(np.isfinite(refs["tlg"]) & (refs["tlg"] < 100.0))))
+    n_tiles = eng.stats()["n_tiles"]
     eng.close()
     tll_chosen = out["tll"].numpy().copy()
     pu = batch.point_updates
     value = whole_job_rate(sum_over_ranks(pg, pu), a.steps, t)
     per_launch_s = float(np.mean(ms)) * 1e-3
     achieved = pu * B_ALG["chosen"] / per_launch_s / 1e9
-    tpp = profiled_traffic(form) if a.config == "munk" else None
+    tpp = profiled_traffic(form, n_tiles) if a.config == "munk" else None
     return {"form": FORM_DESC[form], "precision": form,
             "value": value, "unit": UNIT, "ms_per_step": t / a.steps, **errs,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -549,7 +553,7 @@ def main():
         return 0
     per_launch_s = float(np.mean(march_ms)) * 1e-3
     achieved = pu * B_ALG[a.form] / per_launch_s / 1e9
-    tpp = profiled_traffic(a.form) if a.config == "munk" else None
+    tpp = profiled_traffic(a.form, st["n_tiles"]) if a.config == "munk" else None
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": t_march / a.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,

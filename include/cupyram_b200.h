@@ -57,8 +57,9 @@ enum cr_precision {
                             Pade term and range step: the residual
                             M u - (M + pd2 D) x of the complex64 solve in FP64,
                             its correction solved with the same complex64
-                            factors and added.  Rays on the column kernel or
-                            in the product form run complex128 instead       */
+                            factors and added.  Rays that march on clusters (up
+                            to 6144 rows always) or in the product form run
+                            complex128 instead                                  */
 };
 
 /*
@@ -172,7 +173,7 @@ int cr_pade(double freq, double c0, int np, int ns, double dr, int ip,
 
 /*
  * Pade coefficients of n independent (freq, c0, np, ns, dr, ip) jobs, solved
- * on the current CUDA device, one thread per job, by the same FP64
+ * on the current CUDA device, one warp per job, by the same FP64
  * construction as cr_pade.  Replaces the host loops that call
  * compute_pade_coefficients once per environment and frequency
  * (cupyram/cupyram.py:706-726, :984-999, :1040-1060) and the unused
@@ -229,7 +230,8 @@ int cr_cell_tl(cr_engine* e, int sz, int sr, int ncz, int ncr, float* tl_cells);
 int cr_set_pade(cr_engine* e, int ray, int which, int n, const double* pd1, const double* pd2);
 
 /* Per-ray status flags of the last march (bit 0: non-finite field; bit 1: a
-   bounded wait for the batched march's bulk copies gave up, CR_ETIMEOUT). */
+   bounded wait for the batched march's bulk copies or for a cluster's mailboxes
+   gave up, CR_ETIMEOUT). */
 int cr_ray_flags(cr_engine* e, int32_t* flags, int n);
 
 int cr_get_stats(const cr_engine* e, cr_stats* st);
