@@ -34,7 +34,10 @@
 // shared memory of every CTA (st.async), completing on a barrier of the
 // receiving warp; no CTA waits for a whole cluster.  Two mailboxes alternate:
 // a CTA writes a mailbox again two steps later, after it received the values
-// of the step between, which the reader sent after it had read this one.
+// of the step between, which the reader sent after it had read this one.  A
+// term's mailbox and phase follow from the number of steps that it took part in:
+// the sets of a ray may differ in their number of terms, so a term may sit out
+// steps anywhere in the march.
 // Waits are bounded: one that gives up flags the ray (bit 1).
 //
 // b = M u is a1 (u_{m-1} + 4 u_m + u_{m+1}) with the factor a1 in the stored
@@ -684,10 +687,10 @@ __device__ __forceinline__ void reg_sum(const ColArgs& a, const RegCtx& x, doubl
 
 // One range step of the active set; out >= 0: the step's field is output
 // `out` (outpt.py:11-57; transmission loss follows at the end, reg_tl).
-// step: index of the step, the self-starter's three included.
+// used: steps that this warp's term took part in before.
 template <int L, bool ALL>
 __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int na, const double2 (&al)[L],
-                                         const double2 (&mw)[L], int step, int out) {
+                                         const double2 (&mw)[L], unsigned used, int out) {
     using O = RegOff<L, ALL>;
     constexpr unsigned P16 = 512u * L;  // bytes of a per-row table
     const int k = x.term, l = x.lane, terms = (int)(blockDim.x >> 5);
@@ -745,7 +748,7 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
         double2 e = shfl2_up(h, 1);
         if (l == 0) e = c2(0.0, 0.0);
         // the mailbox of this step: the two alternate over the term's active steps
-        const unsigned count = (unsigned)(k == 0 ? step : step - 2), box = count & 1u, par = (count >> 1) & 1u;
+        const unsigned box = used & 1u, par = (used >> 1) & 1u;
         const unsigned to = x.C > 1 ? remote_addr(tm + O::mail + 512u * box + 32u * (unsigned)x.c,
                                                   (unsigned)min(l, x.C - 1)) : 0u;
         const unsigned to_bar = to - 512u * box - 32u * (unsigned)x.c + (O::bar - O::mail) + 8u * box;
@@ -1011,6 +1014,7 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
     double2 al[L], mw[L];
     const int steps = a.rays[ctl->rid].nr + 3;
     int na = 0, due = ctl->ndr, tlc = 0, stop;
+    int idle = 0;  // steps so far that this warp's term sat out
 #pragma unroll 1
     for (int s = 0; s < steps; s = stop) {
         int want = s == 0 ? 0 : 1;
@@ -1050,8 +1054,9 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
                 if (tlc < ctl->nvr) out = tlc;
                 ++tlc;
             }
-            reg_step<L, ALL>(a, x, na, al, mw, q, out);
+            reg_step<L, ALL>(a, x, na, al, mw, (unsigned)(q - idle), out);
         }
+        if (x.term >= na) idle += stop - s;
     }
     if (threadIdx.x == 0 && ctl->dead) atomicOr(a.flags + ctl->rid, 2);
     __threadfence();

@@ -42,7 +42,8 @@ def load():
         lib = ctypes.CDLL(str(LIB))
         lib.ram_oracle_run.restype = ctypes.c_int
         lib.ram_oracle_run.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
-                                       ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]
+                                       ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
+                                       ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
         lib.ram_oracle_pade.restype = ctypes.c_int
         lib.ram_oracle_pade.argtypes = [ctypes.c_double, ctypes.c_double, ctypes.c_int, ctypes.c_int,
                                         ctypes.c_double, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
@@ -58,8 +59,11 @@ class _Batch(ctypes.Structure):
                 ("grid_len", ctypes.c_int64)]
 
 
-def run(batch, mode="plain", threads=None, rays=None):
-    """March the batch (or the subset of ray indices ``rays``) on the host."""
+def run(batch, mode="plain", threads=None, rays=None, sets=None):
+    """March the batch (or the subset of ray indices ``rays``) on the host.
+
+    sets: {which: (pd1, pd2)}, Pade sets that replace the computed ones of every
+    ray (which as in Engine.set_pade)."""
     lib = load()
     r = np.ascontiguousarray(batch.rays if rays is None else batch.rays[np.asarray(rays)])
     e = np.ascontiguousarray(batch.envs)
@@ -73,9 +77,15 @@ def run(batch, mode="plain", threads=None, rays=None):
     d = _Batch(len(r), len(e), r.ctypes.data, e.ctypes.data, pool.ctypes.data, pool.size, 0,
                1 if batch.compute_grids else 0, line_len, grid_len)
     nthr = threads or os.cpu_count() or 1
+    set_n, set_pd = np.zeros(4, np.int32), np.zeros((2, 4, 10), np.complex128)
+    for which, pair in (sets or {}).items():
+        set_n[which] = len(pair[0])
+        for k in range(2):
+            set_pd[k, which, :len(pair[k])] = pair[k]
     rc = lib.ram_oracle_run(ctypes.byref(d), MODES[mode], tll.ctypes.data, cpl.ctypes.data,
                             tlg.ctypes.data if tlg is not None else None,
-                            cpg.ctypes.data if cpg is not None else None, int(nthr))
+                            cpg.ctypes.data if cpg is not None else None, int(nthr),
+                            set_n.ctypes.data, set_pd[0].ctypes.data, set_pd[1].ctypes.data)
     if rc != 0:
         raise ValueError(f"oracle failed with status {rc} (Pade not converging?)")
     out = {"tll": tll, "cpl": cpl}

@@ -643,7 +643,15 @@ static void outpt(const ray_state* s, const cr_ray* ry, double r, int* mdr, int*
     }
 }
 
-static int run_ray(const cr_batch* b, int ib, int mode, double* tll_all, double* cpl_all,
+/* Pade sets given by the caller instead of computed ones, for every ray: set 0
+   the self-starter's, 1 the ip=2 step's, 2 the march's, 3 the march's without
+   stability constraints; n[w] == 0: set w as computed. */
+typedef struct {
+    int n[4];
+    cd pd1[4][CR_MAX_NP], pd2[4][CR_MAX_NP];
+} oracle_sets;
+
+static int run_ray(const cr_batch* b, int ib, int mode, const oracle_sets* given, double* tll_all, double* cpl_all,
                    double* tlg_all, double* cpg_all) {
     const cr_ray* ry = &b->rays[ib];
     const cr_env* ev = &b->envs[ry->env];
@@ -706,6 +714,17 @@ static int run_ray(const cr_batch* b, int ib, int mode, double* tll_all, double*
     if (oracle_pade(ry->freq, ry->c0, np, ry->ns, ry->dr, 2, sp1, sp2)) rc = -1;
     if (!rc && oracle_pade(ry->freq, ry->c0, np, ry->ns, ry->dr, 1, mp1, mp2)) rc = -1;
     if (rc) { free(dbuf); free(cbuf); return rc; }
+    int n1 = np, n2 = np;
+    if (given && given->n[1]) {
+        n1 = given->n[1];
+        memcpy(sp1, given->pd1[1], sizeof sp1);
+        memcpy(sp2, given->pd2[1], sizeof sp2);
+    }
+    if (given && given->n[2]) {
+        n2 = given->n[2];
+        memcpy(mp1, given->pd1[2], sizeof mp1);
+        memcpy(mp2, given->pd2[2], sizeof mp2);
+    }
 
     profl(&s);
     init_profiles(&s);
@@ -721,23 +740,28 @@ static int run_ray(const cr_batch* b, int ib, int mode, double* tll_all, double*
        remaining np-1 terms with pd = 0 (identity solves); REF mode does too. */
     for (int j = 0; j < CR_MAX_NP; ++j) { pd1[j] = 0.0; pd2[j] = 0.0; }
     pd2[0] = -1.0;
-    const int nself = (mode == ORACLE_REF || mode == ORACLE_SIM) ? np : 1;
+    int nself = (mode == ORACLE_REF || mode == ORACLE_SIM) ? np : 1;
+    if (given && given->n[0]) {
+        nself = given->n[0];
+        memcpy(pd1, given->pd1[0], sizeof pd1);
+        memcpy(pd2, given->pd2[0], sizeof pd2);
+    }
     const int chosen = mode == ORACLE_CHOSEN || mode == ORACLE_CHOSEN_C32 || mode == ORACLE_CHOSEN_F32 ||
                        mode == ORACLE_REFINED;
     const int refine = mode == ORACLE_REFINED;
     const int comb32 = mode == ORACLE_CHOSEN_C32 || mode == ORACLE_CHOSEN_F32, coupling32 = mode == ORACLE_CHOSEN_F32;
     if (chosen) {
-        march_step_chosen(&s, 1, pd1, pd2, comb32, coupling32, refine);
-        march_step_chosen(&s, 1, pd1, pd2, comb32, coupling32, refine);
-        march_step_chosen(&s, np, sp1, sp2, comb32, coupling32, refine);
+        march_step_chosen(&s, nself, pd1, pd2, comb32, coupling32, refine);
+        march_step_chosen(&s, nself, pd1, pd2, comb32, coupling32, refine);
+        march_step_chosen(&s, n1, sp1, sp2, comb32, coupling32, refine);
     } else if (mode == ORACLE_SUM) {
-        march_step_sum(&s, 1, pd1, pd2);
-        march_step_sum(&s, 1, pd1, pd2);
-        march_step_sum(&s, np, sp1, sp2);
+        march_step_sum(&s, nself, pd1, pd2);
+        march_step_sum(&s, nself, pd1, pd2);
+        march_step_sum(&s, n1, sp1, sp2);
     } else {
         march_step(&s, nself, pd1, pd2);
         march_step(&s, nself, pd1, pd2);
-        march_step(&s, np, sp1, sp2);
+        march_step(&s, n1, sp1, sp2);
     }
 
     int mdr = 0, tlc = -1;
@@ -750,12 +774,18 @@ static int run_ray(const cr_batch* b, int ib, int mode, double* tll_all, double*
         if (r >= rs_lim) {
             /* stability constraints off (cupyram.py:976-999) */
             if (oracle_pade(ry->freq, ry->c0, np, 0, ry->dr, 1, mp1, mp2)) { rc = -1; break; }
+            n2 = np;
+            if (given && given->n[3]) {
+                n2 = given->n[3];
+                memcpy(mp1, given->pd1[3], sizeof mp1);
+                memcpy(mp2, given->pd2[3], sizeof mp2);
+            }
             rs_lim = INFINITY;
         }
         init_profiles(&s);
-        if (chosen) march_step_chosen(&s, np, mp1, mp2, comb32, coupling32, refine);
-        else if (mode == ORACLE_SUM) march_step_sum(&s, np, mp1, mp2);
-        else march_step(&s, np, mp1, mp2);
+        if (chosen) march_step_chosen(&s, n2, mp1, mp2, comb32, coupling32, refine);
+        else if (mode == ORACLE_SUM) march_step_sum(&s, n2, mp1, mp2);
+        else march_step(&s, n2, mp1, mp2);
         r = (double)(rn + 2) * s.dr;
         outpt(&s, ry, r, &mdr, &tlc, tll, cpl, tlg, cpg);
     }
@@ -767,6 +797,7 @@ static int run_ray(const cr_batch* b, int ib, int mode, double* tll_all, double*
 typedef struct {
     const cr_batch* b;
     int mode;
+    const oracle_sets* given;
     double *tll, *cpl, *tlg, *cpg;
     int next;
     int err;
@@ -780,7 +811,7 @@ static void* oracle_worker(void* arg) {
         const int ib = job->next++;
         pthread_mutex_unlock(&job->mu);
         if (ib >= job->b->n_rays) break;
-        const int rc = run_ray(job->b, ib, job->mode, job->tll, job->cpl, job->tlg, job->cpg);
+        const int rc = run_ray(job->b, ib, job->mode, job->given, job->tll, job->cpl, job->tlg, job->cpg);
         if (rc) {
             pthread_mutex_lock(&job->mu);
             if (rc < job->err) job->err = rc;
@@ -791,12 +822,22 @@ static void* oracle_worker(void* arg) {
 }
 
 /* Run every ray of the batch on nthreads host threads (one ray per thread at
-   a time).  Returns 0, or the (negative) status of the worst failing ray. */
+   a time).  set_n (NULL, or 4 term counts) with set_pd1 / set_pd2 (4 x CR_MAX_NP
+   complex values each): see oracle_sets.  Returns 0, or the (negative) status
+   of the worst failing ray. */
 int ram_oracle_run(const cr_batch* b, int mode, double* tll, double* cpl, double* tlg, double* cpg,
-                   int nthreads) {
+                   int nthreads, const int* set_n, const double* set_pd1, const double* set_pd2) {
+    oracle_sets given;
+    memset(&given, 0, sizeof given);
+    if (set_n) {
+        memcpy(given.n, set_n, sizeof given.n);
+        memcpy(given.pd1, set_pd1, sizeof given.pd1);
+        memcpy(given.pd2, set_pd2, sizeof given.pd2);
+    }
     oracle_job job;
     job.b = b;
     job.mode = mode;
+    job.given = set_n ? &given : NULL;
     job.tll = tll;
     job.cpl = cpl;
     job.tlg = b->compute_grids ? tlg : NULL;
