@@ -1889,7 +1889,9 @@ int cr_mlp_ensemble_predict(const cr_mlp_net* const* nets, int members, int batc
                             float* spread, int* err, void* stream) {
     if (!nets || members < 1 || members > kMaxMembers || !x || !outs || !mean || !spread) return CR_MLP_EBADSHAPE;
     for (int k = 0; k < members; ++k)
-        if (!nets[k] || !mlp_dims_ok(nets[k], batch)) return CR_MLP_EBADSHAPE;
+        if (!nets[k] || !mlp_dims_ok(nets[k], batch) ||
+            nets[k]->dims[nets[k]->layers] != nets[0]->dims[nets[0]->layers])
+            return CR_MLP_EBADSHAPE;  // the statistics are over outputs of one width
     cudaStream_t st = (cudaStream_t)stream;
     if (!err || !ensemble_fits(nets, members, batch, x, ldx, tc, mean, spread)) {
         for (int k = 0; k < members; ++k) {

@@ -462,8 +462,10 @@ class Ensemble:
         B, n = X.shape[0], len(self.models)
         nets, outs = [], []
         for m in self.models:
-            bufs = m._buffers(B)
             assert X.shape[1] == m.dims[0]
+            if m.dims[-1] != mean.shape[1]:
+                raise ValueError(f"a member has {m.dims[-1]} outputs, the fields have {mean.shape[1]}")
+            bufs = m._buffers(B)
             bufs[0][0] = X
             nets.append(m._net(B, w16=m.Wb, b=m.b))
             outs.append(bufs[1].data_ptr())

@@ -113,7 +113,8 @@ int cr_mlp_ensemble_stats(const float* const* preds, int members, long long n, f
 /* The ensemble's forward passes for x (bf16, row stride ldx) and their
  * statistics, as cr_mlp_forward of every member and cr_mlp_ensemble_stats give
  * them; mean and spread are [batch][dims[layers]].  nets: host array of
- * `members` networks (w16, b and act are used).  Two to four members of one
+ * `members` networks (w16, b and act are used), all with as many outputs
+ * (CR_MLP_EBADSHAPE otherwise).  Two to four members of one
  * shape, all of it on the tcgen05 kernel, take one launch a hidden layer and one
  * for the output layers with the statistics; outs[k] is then left as it was.
  * Otherwise outs[k] (16-byte aligned) holds member k's outputs. */
