@@ -1786,6 +1786,10 @@ int cr_mlp_backward(const cr_mlp_net* net, int batch, const void* x, int ldx, in
     if (!mlp_dims_ok(net, batch) || !x || ldx % 8 || !aligned16(x)) return CR_MLP_EBADSHAPE;
     cudaStream_t st = (cudaStream_t)stream;
     const int L = net->layers;
+    for (int l = 0; l < L; ++l)  // transpose_mats moves 16 bytes at a time
+        if (!aligned16(net->grad[l]) || !aligned16(net->grad_t[l]) || !aligned16(net->act_t[l]) ||
+            (l > 0 && !aligned16(net->act[l])))
+            return CR_MLP_EBADSHAPE;
     // gradients down to the first layer's output, through the ReLU whose output was act[l]
     for (int l = L - 1; l > 0; --l) {
         const int rc = mlp_gemm_any(CR_MLP_EPI_RELU_MASK_BF16, tc, net->grad[l], net->wt16[l], batch, net->dims[l],
@@ -1836,7 +1840,21 @@ int cr_mlp_step(const cr_mlp_net* net, float lr, float beta1, float beta2, float
     for (int l0 = 0; l0 < net->layers; l0 += kMaxMats / 2) {
         AdamMats t{};
         for (int l = l0; l < net->layers && l < l0 + kMaxMats / 2; ++l) {
-            const int w = t.n, b = w + 1, d_out = net->dims[l + 1], d_in = net->dims[l];
+            const int d_out = net->dims[l + 1], d_in = net->dims[l];
+            // the fused kernel moves 16 bytes at a time; matrices that start elsewhere go
+            // through the single-matrix calls
+            if (!aligned16(net->w[l]) || !aligned16(net->gw[l]) || !aligned16(net->mw[l]) || !aligned16(net->vw[l]) ||
+                !aligned16(net->w16[l]) || !aligned16(net->wt16[l])) {
+                int rc = cr_mlp_adam(net->w[l], net->gw[l], net->mw[l], net->vw[l], net->w16[l], (long long)d_out * d_in,
+                                     lr, beta1, beta2, eps, step, weight_decay, stream);
+                if (!rc) rc = cr_mlp_transpose(net->w16[l], d_in, net->wt16[l], d_out, d_out, d_in, stream);
+                if (!rc)
+                    rc = cr_mlp_adam(net->b[l], net->gb[l], net->mb[l], net->vb[l], nullptr, d_out, lr, beta1, beta2, eps,
+                                     step, 0.f, stream);
+                if (rc) return rc;
+                continue;
+            }
+            const int w = t.n, b = w + 1;
             t.n += 2;
             t.p[w] = net->w[l];
             t.g[w] = net->gw[l];
@@ -1855,6 +1873,7 @@ int cr_mlp_step(const cr_mlp_net* net, float lr, float beta1, float beta2, float
             t.cols[b] = 1;
             t.first[b + 1] = t.first[b] + (d_out + 4095) / 4096;
         }
+        if (t.n == 0) continue;
         if (launch_next(adam_mats, dim3(t.first[t.n]), dim3(256), 0, (cudaStream_t)stream, t,
                         adam_args(lr, beta1, beta2, eps, step), weight_decay) != cudaSuccess)
             return CR_MLP_ECUDA;

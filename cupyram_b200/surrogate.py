@@ -180,6 +180,12 @@ def transpose(src, dst):
 # ---------------------------------------------------------------------------
 # the MLP
 # ---------------------------------------------------------------------------
+def _dense(*lists):
+    """The whole-network calls take dense matrices; a user's own (a column range of a wider
+    matrix, say) go layer by layer, through calls that take row strides."""
+    return all(t.is_contiguous() for lst in lists for t in lst)
+
+
 class MLP:
     """Fully connected ReLU network in BF16 with FP32 accumulation and FP32
     master weights; dims = [d_in, hidden..., d_out], all multiples of 128."""
@@ -243,6 +249,11 @@ class MLP:
         H, out, _, _, _ = self._buffers(B)
         assert X.shape[1] == self.dims[0]
         H[0] = X
+        if not _dense(self.Wb):
+            for l, w in enumerate(self.Wb[:-1]):
+                gemm(EPI_BIAS_RELU_BF16, H[l], w, H[l + 1], bias=self.b[l])
+            gemm(EPI_BIAS_F32, H[-1], self.Wb[-1], out, bias=self.b[-1])
+            return out
         _ok(kernels().cr_mlp_forward(self._net(B, w16=self.Wb, b=self.b), B, _p(X), X.stride(0), _p(out),
                                      int(USE_TCGEN05), _p(tc_error_flag()), _stream()), "cr_mlp_forward")
         return out
@@ -250,15 +261,38 @@ class MLP:
     def backward(self, dout):
         """dout: [B, d_out] bf16 gradient of the loss at the output; fills gW, gb."""
         B = dout.shape[0]
-        H, _, dH, _, _ = self._buffers(B)
+        H, _, dH, T, T2 = self._buffers(B)
         if dH[-1].data_ptr() != dout.data_ptr():
             dH[-1].copy_(dout)
         X = H[0]
+        if not _dense(self.WTb, self.gW):
+            for l in range(len(self.W) - 1, -1, -1):
+                transpose(dH[l], T[l])
+                transpose(H[l], T2[l])
+                gemm(EPI_F32, T[l], T2[l], self.gW[l])
+                _ok(kernels().cr_mlp_col_sum(_p(dH[l]), dH[l].stride(0), B, dH[l].shape[1], _p(self.gb[l]),
+                                             _stream()), "cr_mlp_col_sum")
+                if l > 0:
+                    gemm(EPI_RELU_MASK_BF16, dH[l], self.WTb[l], dH[l - 1], mask=H[l])
+            return
         _ok(kernels().cr_mlp_backward(self._net(B, wt16=self.WTb, gw=self.gW, gb=self.gb), B, _p(X), X.stride(0),
                                       int(USE_TCGEN05), _p(tc_error_flag()), _stream()), "cr_mlp_backward")
 
     def step(self, lr, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
         self.t += 1
+        if not _dense(self.W, self.gW, self.mW, self.vW, self.Wb, self.WTb):
+            for l in range(len(self.W)):
+                for mine, wd in (((self.W, self.gW, self.mW, self.vW, self.Wb), weight_decay),
+                                 ((self.b, self.gb, self.mb, self.vb, None), 0.0)):
+                    own = [t[l] if t else None for t in mine]
+                    dense = [t.contiguous() if t is not None else None for t in own]
+                    _ok(kernels().cr_mlp_adam(*map(_p, dense), own[0].numel(), lr, beta1, beta2, eps, self.t, wd,
+                                              _stream()), "cr_mlp_adam")
+                    for t, d in zip(own, dense):
+                        if d is not t:
+                            t.copy_(d)
+                transpose(self.Wb[l], self.WTb[l])
+            return
         net = self._net(w=self.W, b=self.b, w16=self.Wb, wt16=self.WTb, gw=self.gW, gb=self.gb, mw=self.mW,
                         vw=self.vW, mb=self.mb, vb=self.vb)
         _ok(kernels().cr_mlp_step(net, lr, beta1, beta2, eps, self.t, weight_decay, _stream()), "cr_mlp_step")
@@ -484,7 +518,7 @@ class Ensemble:
         spread = torch.empty(n, NZ_OUT * NR_OUT, device=X.device)
         for s in range(0, n, chunk):
             xb = X[s: s + chunk]
-            if len(self.models) <= MAX_MEMBERS:
+            if len(self.models) <= MAX_MEMBERS and all(_dense(m.Wb) for m in self.models):
                 self._predict_chunk(xb, mean[s: s + chunk], spread[s: s + chunk])
                 continue
             preds = [m.forward(xb) for m in self.models]

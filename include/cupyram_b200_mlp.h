@@ -70,7 +70,8 @@ int cr_mlp_adam(float* p, const float* g, float* m, float* v, void* p_bf16, long
 /* A fully connected ReLU network of `layers` layers, dims[0] inputs to
  * dims[layers] outputs (all multiples of 128), as the three calls below take
  * it: host arrays of device pointers, one per layer l, matrices row-major and
- * dense.  Arrays that a call does not use may be NULL. */
+ * dense, act, grad, act_t and grad_t 16-byte aligned (cr_mlp_backward:
+ * CR_MLP_EBADSHAPE otherwise).  Arrays that a call does not use may be NULL. */
 typedef struct cr_mlp_net {
     int layers;
     const int* dims;      /* [layers + 1]                                       */

@@ -37,6 +37,6 @@ def test_predict_refuses_members_of_another_field_size(d_out):
     never accepted, and would be written past the results' end."""
     torch = pytest.importorskip("torch")
     ens = S.Ensemble.__new__(S.Ensemble)
-    ens.models = [SimpleNamespace(dims=[S.D_IN, d_out]) for _ in range(2)]
+    ens.models = [SimpleNamespace(dims=[S.D_IN, d_out], Wb=[]) for _ in range(2)]
     with pytest.raises(ValueError, match="outputs"):
         ens.predict(torch.zeros(128, S.D_IN, dtype=torch.bfloat16), check=False)
