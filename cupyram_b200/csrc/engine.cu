@@ -46,7 +46,6 @@
 #include <mutex>
 #include <numeric>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <tuple>
 #include <vector>
@@ -58,6 +57,7 @@
 #include "march_sum.cuh"
 #include "pade.h"
 #include "pade_warp.cuh"
+#include "staging.h"
 
 namespace {
 
@@ -773,126 +773,6 @@ void free_all(cr_engine* e) {
     lane_give(e->device, {e->stream, e->ev_fork});
     for (auto& ev : e->ev)
         if (ev) cudaEventDestroy(ev);
-}
-
-// Pinned staging of host-to-device copies.  A pageable cudaMemcpy is staged
-// by the driver through its own pinned buffers, one host copy at a time; here
-// each device has a ring of two pinned chunks, allocated once: while one
-// chunk's DMA runs, host threads fill the other, so the host copy and the
-// transfer overlap and the copy itself runs on several cores.
-constexpr size_t kStageChunk = 16u << 20;  // bytes per chunk
-constexpr size_t kStageMin = 4u << 20;     // smaller copies go direct
-constexpr int kStageThreads = 4;
-struct StageRing {
-    unsigned char* buf[2] = {nullptr, nullptr};
-    cudaEvent_t done[2] = {nullptr, nullptr};
-    cudaEvent_t out[32] = {};  // staged_d2h: one per piece
-};
-StageRing g_stage[kPoolDevices];
-std::mutex g_stage_mu[kPoolDevices];
-
-void copy_parallel(unsigned char* dst, const unsigned char* src, size_t n) {
-    if (n < (1u << 20)) {
-        memcpy(dst, src, n);
-        return;
-    }
-    std::thread th[kStageThreads - 1];
-    const size_t part = (n / kStageThreads + 63) & ~size_t(63);
-    for (int t = 1; t < kStageThreads; ++t) {
-        const size_t lo = std::min(n, part * t), hi = std::min(n, part * (t + 1));
-        th[t - 1] = std::thread([=] { memcpy(dst + lo, src + lo, hi - lo); });
-    }
-    memcpy(dst, src, std::min(n, part));
-    for (auto& x : th) x.join();
-}
-
-// Host-to-device copy of `bytes` through the device's pinned ring, ordered on
-// `st`.  Returns when the last chunk's copy has been queued (the caller
-// synchronises the stream); the ring is held until then.
-cudaError_t staged_h2d(int dev, void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (dev < 0 || dev >= kPoolDevices) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lock(g_stage_mu[dev]);
-    StageRing& R = g_stage[dev];
-    cudaError_t ce = cudaSuccess;
-    for (int k = 0; k < 2 && ce == cudaSuccess; ++k) {
-        if (!R.buf[k]) ce = cudaHostAlloc((void**)&R.buf[k], kStageChunk, cudaHostAllocPortable);
-        if (ce == cudaSuccess && !R.done[k]) ce = cudaEventCreateWithFlags(&R.done[k], cudaEventDisableTiming);
-    }
-    const unsigned char* s = (const unsigned char*)src;
-    unsigned char* d = (unsigned char*)dst;
-    int k = 0;
-    for (size_t off = 0; off < bytes && ce == cudaSuccess; off += kStageChunk, k ^= 1) {
-        const size_t n = std::min(kStageChunk, bytes - off);
-        ce = cudaEventSynchronize(R.done[k]);  // the chunk's previous DMA has finished
-        if (ce != cudaSuccess) break;
-        copy_parallel(R.buf[k], s + off, n);
-        ce = cudaMemcpyAsync(d + off, R.buf[k], n, cudaMemcpyHostToDevice, st);
-        if (ce == cudaSuccess) ce = cudaEventRecord(R.done[k], st);
-    }
-    // the ring is reused by the next call only after these copies: wait for them
-    for (int j = 0; j < 2 && ce == cudaSuccess; ++j) ce = cudaEventSynchronize(R.done[j]);
-    return ce;
-}
-
-// Device-to-host copy of `bytes` into pageable memory through the same ring, in
-// pieces of 1 MB: their DMAs are queued at once and host threads copy each piece
-// out as it arrives.  The driver's own staging copies on one thread, which for a
-// freshly allocated result spends its time on page faults (12 MB: 3.9 ms, here
-// 1.9 ms).  Returns with the copy complete.
-constexpr size_t kOutPiece = 1u << 20;
-constexpr size_t kOutMin = 2u << 20;  // smaller copies go direct
-constexpr int kOutThreads = 6;
-constexpr int kOutPieces = (int)(2 * kStageChunk / kOutPiece);
-static_assert(kOutPieces <= 32, "an event per piece");
-cudaError_t staged_d2h(int dev, void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (dev < 0 || dev >= kPoolDevices) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lock(g_stage_mu[dev]);
-    StageRing& R = g_stage[dev];
-    cudaError_t ce = cudaSuccess;
-    for (int k = 0; k < 2 && ce == cudaSuccess; ++k) {
-        if (!R.buf[k]) ce = cudaHostAlloc((void**)&R.buf[k], kStageChunk, cudaHostAllocPortable);
-        if (ce == cudaSuccess && !R.done[k]) ce = cudaEventCreateWithFlags(&R.done[k], cudaEventDisableTiming);
-    }
-    for (int k = 0; k < kOutPieces && ce == cudaSuccess; ++k)
-        if (!R.out[k]) ce = cudaEventCreateWithFlags(&R.out[k], cudaEventDisableTiming);
-    for (int k = 0; k < 2 && ce == cudaSuccess; ++k) ce = cudaEventSynchronize(R.done[k]);
-    auto piece = [&](int k) { return R.buf[k / (kOutPieces / 2)] + (size_t)(k % (kOutPieces / 2)) * kOutPiece; };
-    for (size_t off = 0; off < bytes && ce == cudaSuccess; off += 2 * kStageChunk) {
-        const size_t span = std::min(2 * kStageChunk, bytes - off);
-        const int n = (int)((span + kOutPiece - 1) / kOutPiece);
-        auto size = [&](int k) { return std::min(kOutPiece, span - (size_t)k * kOutPiece); };
-        int queued = 0;
-        for (; queued < n && ce == cudaSuccess; ++queued) {
-            ce = cudaMemcpyAsync(piece(queued), (const unsigned char*)src + off + (size_t)queued * kOutPiece,
-                                 size(queued), cudaMemcpyDeviceToHost, st);
-            if (ce == cudaSuccess) ce = cudaEventRecord(R.out[queued], st);
-        }
-        std::atomic<int> turn{0}, failed{(int)cudaSuccess};
-        auto work = [&] {
-            for (int k = turn++; k < n; k = turn++) {
-                const cudaError_t e = cudaEventSynchronize(R.out[k]);
-                if (e != cudaSuccess) {
-                    failed = (int)e;
-                    return;
-                }
-                memcpy((unsigned char*)dst + off + (size_t)k * kOutPiece, piece(k), size(k));
-            }
-        };
-        if (ce == cudaSuccess) {
-            std::thread th[kOutThreads - 1];
-            try {
-                for (int t = 0; t + 1 < std::min(n, kOutThreads); ++t) th[t] = std::thread(work);
-            } catch (const std::system_error&) {
-                // no more threads to be had: those that run and this one do the work
-            }
-            work();
-            for (auto& x : th)
-                if (x.joinable()) x.join();
-            ce = (cudaError_t)failed.load();
-        }
-        if (ce != cudaSuccess) cudaStreamSynchronize(st);  // no DMA still writes the ring
-    }
-    return ce;
 }
 
 // Validate the batch; returns an error message or empty string.
@@ -1874,7 +1754,7 @@ int cr_upload(cr_engine* e) {
         if (ce != cudaSuccess || !bytes) return;
         // large arrays (the environment pool) go through the pinned staging
         // ring; small tables are copied directly
-        ce = bytes >= kStageMin ? staged_h2d(e->device, dst, src, bytes, e->stream)
+        ce = bytes >= crk::kStageMin ? crk::staged_h2d(e->device, dst, src, bytes, e->stream)
                                 : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->stream);
     };
     cp(e->d_rays, e->rays.data(), e->rays.size() * sizeof(RayDev));
@@ -2084,12 +1964,12 @@ int cr_download(cr_engine* e, const cr_outputs* out) {
     if (ce == cudaSuccess) ce = cudaEventRecord(e->ev[2], e->stream);
     auto cp = [&](void* dst, const void* src, size_t n) {
         if (ce == cudaSuccess && n && dst) {
-            bool pageable = n >= kOutMin;
+            bool pageable = n >= crk::kOutMin;
             if (pageable) {
                 cudaPointerAttributes at{};
                 pageable = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
             }
-            ce = pageable ? staged_d2h(e->device, dst, src, n, e->stream)
+            ce = pageable ? crk::staged_d2h(e->device, dst, src, n, e->stream)
                           : cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, e->stream);
             bytes += (long long)n;
         }
