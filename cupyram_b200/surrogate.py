@@ -183,7 +183,11 @@ def transpose(src, dst):
 def _dense(*lists):
     """The whole-network calls take dense matrices; a user's own (a column range of a wider
     matrix, say) go layer by layer, through calls that take row strides."""
-    return all(t.is_contiguous() for lst in lists for t in lst)
+    for lst in lists:
+        for t in lst:
+            if not t.is_contiguous():
+                return False
+    return True
 
 
 class MLP:
@@ -254,7 +258,7 @@ class MLP:
                 gemm(EPI_BIAS_RELU_BF16, H[l], w, H[l + 1], bias=self.b[l])
             gemm(EPI_BIAS_F32, H[-1], self.Wb[-1], out, bias=self.b[-1])
             return out
-        _ok(kernels().cr_mlp_forward(self._net(B, w16=self.Wb, b=self.b), B, _p(X), X.stride(0), _p(out),
+        _ok(kernels().cr_mlp_forward(self._net(w16=self.Wb, b=self.b, act=H), B, _p(X), X.stride(0), _p(out),
                                      int(USE_TCGEN05), _p(tc_error_flag()), _stream()), "cr_mlp_forward")
         return out
 
@@ -493,15 +497,15 @@ class Ensemble:
         return losses
 
     def _predict_chunk(self, X, mean, spread):
-        B, n = X.shape[0], len(self.models)
+        (B, d_in), n, width = X.shape, len(self.models), mean.shape[1]
         nets, outs = [], []
         for m in self.models:
-            assert X.shape[1] == m.dims[0]
-            if m.dims[-1] != mean.shape[1]:
-                raise ValueError(f"a member has {m.dims[-1]} outputs, the fields have {mean.shape[1]}")
+            assert d_in == m.dims[0]
+            if m.dims[-1] != width:
+                raise ValueError(f"a member has {m.dims[-1]} outputs, the fields have {width}")
             bufs = m._buffers(B)
             bufs[0][0] = X
-            nets.append(m._net(B, w16=m.Wb, b=m.b))
+            nets.append(m._net(w16=m.Wb, b=m.b, act=bufs[0]))
             outs.append(bufs[1].data_ptr())
         _ok(kernels().cr_mlp_ensemble_predict((ctypes.c_void_p * n)(*[ctypes.addressof(t) for t in nets]), n, B, _p(X),
                                               X.stride(0), (ctypes.c_void_p * n)(*outs), int(USE_TCGEN05), TL_SCALE,
@@ -518,7 +522,7 @@ class Ensemble:
         spread = torch.empty(n, NZ_OUT * NR_OUT, device=X.device)
         for s in range(0, n, chunk):
             xb = X[s: s + chunk]
-            if len(self.models) <= MAX_MEMBERS and all(_dense(m.Wb) for m in self.models):
+            if len(self.models) <= MAX_MEMBERS and _dense(*[m.Wb for m in self.models]):
                 self._predict_chunk(xb, mean[s: s + chunk], spread[s: s + chunk])
                 continue
             preds = [m.forward(xb) for m in self.models]
