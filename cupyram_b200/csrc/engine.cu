@@ -51,6 +51,7 @@
 #include <vector>
 
 #include "../../include/cupyram_b200.h"
+#include "lanes.h"
 #include "march_col.cuh"
 #include "march_reg.cuh"
 #include "march_common.cuh"
@@ -643,6 +644,7 @@ struct cr_engine {
     cudaEvent_t ev_fork = nullptr;
     long long device_bytes = 0;
     bool uploaded = false, marched = false;
+    bool joined = true;  // no stream holds work that the engine's own has not waited for
     cr_stats st{};
 
     int fail(int code, const char* fmt, ...) {
@@ -695,46 +697,7 @@ cudaError_t engine_pool(int dev, cudaMemPool_t* out) {
     return cudaSuccess;
 }
 
-// Streams (with an event each) of the engines' launches, kept for the next
-// engine: creating and destroying one costs about 70 us, and an uneven batch
-// takes dozens.  At most kLanesKept idle ones per device; cr_release_cache
-// destroys them.  A lane is given back idle.
-struct StreamLane {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t done = nullptr;
-};
-constexpr size_t kLanesKept = 128;
-std::vector<StreamLane> g_lanes[kPoolDevices];
-std::mutex g_lanes_mu;
-
-cudaError_t lane_take(int dev, StreamLane* out) {
-    if (dev >= 0 && dev < kPoolDevices) {
-        std::lock_guard<std::mutex> lock(g_lanes_mu);
-        if (!g_lanes[dev].empty()) {
-            *out = g_lanes[dev].back();
-            g_lanes[dev].pop_back();
-            return cudaSuccess;
-        }
-    }
-    StreamLane l;
-    cudaError_t ce = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
-    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming);
-    if (ce != cudaSuccess && l.stream) cudaStreamDestroy(l.stream);
-    else *out = l;
-    return ce;
-}
-void lane_give(int dev, StreamLane l) {
-    if (!l.stream) return;
-    if (dev >= 0 && dev < kPoolDevices) {
-        std::lock_guard<std::mutex> lock(g_lanes_mu);
-        if (g_lanes[dev].size() < kLanesKept) {
-            g_lanes[dev].push_back(l);
-            return;
-        }
-    }
-    cudaEventDestroy(l.done);
-    cudaStreamDestroy(l.stream);
-}
+crk::LanePool g_lanes;
 
 template <typename T>
 cudaError_t dev_alloc(cr_engine* e, T** p, size_t count) {
@@ -754,23 +717,23 @@ void free_all(cr_engine* e) {
                     e->d_S3,   e->d_AL,   e->d_WF,   e->d_tile_G,  e->d_tile_off, e->d_tile_loff, e->d_pfc, e->d_pfcinf,
                     e->d_QD,   e->d_WD,   e->d_QU,   e->d_WU,      e->d_ED,  e->d_EU, e->d_col_ray,
                     e->d_queue, e->d_ticket, e->d_E2};
-    // stream-ordered frees on the engine's stream (every other stream of the
-    // engine joins it at the end of each march), back into the pool
-    if (e->stream) {
-        for (void* p : ptrs)
-            if (p) cudaFreeAsync(p, e->stream);
-        cudaStreamSynchronize(e->stream);
-    }
-    // a march that failed half way may have left work on streams that never joined
-    if (!e->marched) {
+    // every other stream of the engine joins its own at the end of a march, but not
+    // when the march failed half way: nothing may still use the memory then
+    if (!e->joined) {
         for (auto& g : e->col_groups)
             if (g.stream) cudaStreamSynchronize(g.stream);
         for (size_t i = 1; i < e->sum_streams.size(); ++i)
             if (e->sum_streams[i]) cudaStreamSynchronize(e->sum_streams[i]);
     }
-    for (auto& g : e->col_groups) lane_give(e->device, {g.stream, g.done});
-    for (size_t i = 1; i < e->sum_streams.size(); ++i) lane_give(e->device, {e->sum_streams[i], e->sum_done[i]});
-    lane_give(e->device, {e->stream, e->ev_fork});
+    // stream-ordered frees on the engine's stream, back into the pool
+    if (e->stream) {
+        for (void* p : ptrs)
+            if (p) cudaFreeAsync(p, e->stream);
+        cudaStreamSynchronize(e->stream);
+    }
+    for (auto& g : e->col_groups) g_lanes.give(e->device, {g.stream, g.done});
+    for (size_t i = 1; i < e->sum_streams.size(); ++i) g_lanes.give(e->device, {e->sum_streams[i], e->sum_done[i]});
+    g_lanes.give(e->device, {e->stream, e->ev_fork});
     for (auto& ev : e->ev)
         if (ev) cudaEventDestroy(ev);
 }
@@ -862,9 +825,9 @@ cudaError_t device_pade(const std::vector<PadeJob>& jobs, std::vector<double2>& 
     status.assign((size_t)n, CR_OK);
     if (n == 0) return cudaSuccess;
     int dev = 0;
-    StreamLane lane;
+    crk::StreamLane lane;
     cudaError_t ce = cudaGetDevice(&dev);
-    if (ce == cudaSuccess) ce = lane_take(dev, &lane);
+    if (ce == cudaSuccess) ce = g_lanes.take(dev, &lane);
     if (ce != cudaSuccess) return ce;
     cudaStream_t st = lane.stream;
     // regions rounded up to 256 bytes: the coefficient arrays are double2 and
@@ -897,7 +860,7 @@ cudaError_t device_pade(const std::vector<PadeJob>& jobs, std::vector<double2>& 
     }
     const cudaError_t cs = cudaStreamSynchronize(st);
     if (ce == cudaSuccess) ce = cs;
-    lane_give(dev, lane);
+    g_lanes.give(dev, lane);
     return ce;
 }
 
@@ -1633,8 +1596,8 @@ int cr_create(const cr_batch* b, cr_engine** out) {
 
     cudaError_t ce = cudaGetDevice(&e->device);
     if (ce == cudaSuccess) {
-        StreamLane l;
-        ce = lane_take(e->device, &l);
+        crk::StreamLane l;
+        ce = g_lanes.take(e->device, &l);
         e->stream = l.stream;
         e->ev_fork = l.done;
     }
@@ -1677,16 +1640,16 @@ int cr_create(const cr_batch* b, cr_engine** out) {
             e->sum_done.assign(e->sum_streams.size(), nullptr);
             e->sum_streams[0] = e->stream;
             for (size_t i = 1; i < e->sum_streams.size() && ce == cudaSuccess; ++i) {
-                StreamLane l;
-                ce = lane_take(e->device, &l);
+                crk::StreamLane l;
+                ce = g_lanes.take(e->device, &l);
                 e->sum_streams[i] = l.stream;
                 e->sum_done[i] = l.done;
             }
         }
         for (auto& g : e->col_groups) {
             if (ce != cudaSuccess) break;
-            StreamLane l;
-            ce = lane_take(e->device, &l);
+            crk::StreamLane l;
+            ce = g_lanes.take(e->device, &l);
             g.stream = l.stream;
             g.done = l.done;
         }
@@ -1790,6 +1753,7 @@ int cr_march(cr_engine* e) {
     if (!e) return CR_EINVAL;
     if (!e->uploaded) return e->fail(CR_ESTATE, "cr_march: call cr_upload first");
     cudaError_t ce = cudaSetDevice(e->device);
+    e->joined = false;  // until every launch below has ended
     MarchArgs a;
     a.rays = e->d_rays;
     a.tile_ray = e->d_tile_ray;
@@ -1935,6 +1899,7 @@ int cr_march(cr_engine* e) {
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]);
     if (ce != cudaSuccess) return e->cuda_fail(ce, "cr_march");
+    e->joined = true;
     e->st.march_ms = ms;
     if (!e->sum_mode) e->st.kernel_launches = 1;
     std::vector<int> fl(e->n_rays);
@@ -2230,14 +2195,7 @@ int cr_release_cache(void) {
             return CR_ECUDA;
         }
     }
-    std::lock_guard<std::mutex> lanes(g_lanes_mu);
-    for (int d = 0; d < kPoolDevices; ++d) {
-        for (const StreamLane& l : g_lanes[d]) {
-            cudaEventDestroy(l.done);
-            cudaStreamDestroy(l.stream);
-        }
-        g_lanes[d].clear();
-    }
+    g_lanes.clear();
     return CR_OK;
 }
 

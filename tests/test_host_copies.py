@@ -44,3 +44,36 @@ int main() {
 }
 """)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_lanes_are_idle_when_they_are_taken_again(tmp_path):
+    """A lane given back with work still on it (an engine whose march failed between its
+    launches) is not handed on before that work is done; the pool keeps a bounded number
+    per device, hands out a device's own, and clear destroys them."""
+    r = _run(tmp_path, r"""
+#include "lanes.h"
+#include <cstdio>
+int main() {
+    crk::LanePool pool;
+    crk::StreamLane l, m;
+    char a[4] = "abc", b[4] = "";
+    cudaSetDevice(2);
+    if (pool.take(2, &l) != cudaSuccess) return 1;
+    cudaMemcpyAsync(b, a, 4, cudaMemcpyHostToDevice, l.stream);  // never waited for
+    pool.give(2, l);
+    if (pool.take(2, &m) != cudaSuccess || m.stream != l.stream) return 2;
+    if (!m.stream->work.empty() || b[0] != 'a') return printf("a busy lane was handed on\n"), 3;
+    pool.give(2, m);
+    cudaSetDevice(1);
+    if (pool.take(1, &l) != cudaSuccess || l.stream == m.stream || l.stream->device != 1) return 4;
+    std::vector<crk::StreamLane> many(crk::LanePool::kKept + 20);
+    for (auto& x : many) pool.take(1, &x);
+    for (auto& x : many) pool.give(1, x);
+    pool.give(1, l);
+    if (fake::streams_alive != (int)crk::LanePool::kKept + 1) return 5;
+    pool.clear();
+    if (fake::streams_alive) return 6;
+    return 0;
+}
+""")
+    assert r.returncode == 0, r.stdout + r.stderr
