@@ -849,8 +849,14 @@ __device__ __forceinline__ int mat_of(const Mats& t, int block) {
 // of 512: 158 -> 153 us).
 __device__ __forceinline__ int tile_place(int c, int r) { return (((r >> 3) ^ (c >> 3)) & 7) * 8 + (r & 7); }
 
+// A transposed tile; its rows are read and written 16 bytes at a time.
+struct __align__(16) Tile64 {
+    __nv_bfloat16 v[64][72];
+};
+static_assert(alignof(Tile64) >= 16 && sizeof(Tile64) % (64 * 16) == 0, "rows on 16-byte boundaries");
+
 __global__ void __launch_bounds__(256) transpose_mats(const __grid_constant__ Mats t) {
-    __shared__ __nv_bfloat16 tile[64][72];
+    __shared__ Tile64 tile;
     const int i = mat_of(t, blockIdx.x), b = blockIdx.x - t.first[i], nc = t.cols[i] / 64;
     const int r0 = (b / nc) * 64, c0 = (b % nc) * 64;
     const __nv_bfloat16* src = t.src[i];
@@ -861,13 +867,13 @@ __global__ void __launch_bounds__(256) transpose_mats(const __grid_constant__ Ma
         const uint4 v = *reinterpret_cast<const uint4*>(src + (size_t)(r0 + r) * t.lds[i] + c0 + c);
         const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) tile[c + j][tile_place(c, r)] = e[j];
+        for (int j = 0; j < 8; ++j) tile.v[c + j][tile_place(c, r)] = e[j];
     }
     __syncthreads();
     for (int q = threadIdx.x; q < 512; q += 256) {
         const int c = q >> 3, r = (q & 7) * 8;
         *reinterpret_cast<uint4*>(dst + (size_t)(c0 + c) * t.ldd[i] + r0 + r) =
-            *reinterpret_cast<const uint4*>(&tile[c][tile_place(c, r)]);
+            *reinterpret_cast<const uint4*>(&tile.v[c][tile_place(c, r)]);
     }
 }
 
@@ -992,7 +998,7 @@ struct AdamMats {
 };
 __global__ void __launch_bounds__(256) adam_mats(const __grid_constant__ AdamMats t, AdamArgs a, float wd) {
     launch_order();
-    __shared__ __nv_bfloat16 tile[64][72];
+    __shared__ Tile64 tile;
     int i = 0;
     while ((int)blockIdx.x >= t.first[i + 1]) ++i;
     const int b = blockIdx.x - t.first[i];
@@ -1024,16 +1030,16 @@ __global__ void __launch_bounds__(256) adam_mats(const __grid_constant__ AdamMat
         __nv_bfloat162 w[2] = {__floats2bfloat162_rn(p.x, p.y), __floats2bfloat162_rn(p.z, p.w)};
         *reinterpret_cast<uint2*>(t.pb[i] + o) = *reinterpret_cast<const uint2*>(w);
         const int at = tile_place(c, r);
-        tile[c][at] = w[0].x;
-        tile[c + 1][at] = w[0].y;
-        tile[c + 2][at] = w[1].x;
-        tile[c + 3][at] = w[1].y;
+        tile.v[c][at] = w[0].x;
+        tile.v[c + 1][at] = w[0].y;
+        tile.v[c + 2][at] = w[1].x;
+        tile.v[c + 3][at] = w[1].y;
     }
     __syncthreads();
     for (int q = threadIdx.x; q < 512; q += 256) {
         const int c = q >> 3, r = (q & 7) * 8;
         *reinterpret_cast<uint4*>(t.pt[i] + (size_t)(c0 + c) * t.rows[i] + r0 + r) =
-            *reinterpret_cast<const uint4*>(&tile[c][tile_place(c, r)]);
+            *reinterpret_cast<const uint4*>(&tile.v[c][tile_place(c, r)]);
     }
 }
 
