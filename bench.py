@@ -573,6 +573,8 @@ def main():
                              "calls": "cr_run on an engine already created (upload, march, download)"},
             "gpu_launches": int(launches), "clocks": clk.summary(),
             "schedule": {"column_rays": int(st["column_rays"]), "column_launches": int(st["column_launches"]),
+                         "cluster_rays": int(st["cluster_rays"]), "cluster_launches": int(st["cluster_launches"]),
+                         "cluster_register_rays": int(st["cluster_register_rays"]),
                          "queue_ctas": int(st["queue_ctas"]), "tuner_row_step_s": st["tuner_row_step_s"],
                          "tuner_updates_per_s": st["tuner_updates_per_s"], "tuner_slots": st["tuner_slots"],
                          "create_ms": st["create_ms"], "pade_ms": st["pade_ms"]}}

@@ -60,6 +60,10 @@ class CrStats(ctypes.Structure):
                 ("tuner_slots", ctypes.c_double)]
 
 
+class CrClusterStats(ctypes.Structure):
+    _fields_ = [(k, ctypes.c_int32) for k in ("rays", "register_rays", "launches", "register_launches")]
+
+
 # every symbol the header declares, with its signature
 _SIGS = {
     "cr_abi_version": (ctypes.c_int, []),
@@ -75,6 +79,7 @@ _SIGS = {
                                    ctypes.c_void_p, ctypes.c_void_p]),
     "cr_ray_flags": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]),
     "cr_get_stats": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(CrStats)]),
+    "cr_get_cluster_stats": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(CrClusterStats)]),
     "cr_last_error": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_size_t]),
     "cr_global_error": (ctypes.c_int, [ctypes.c_char_p, ctypes.c_size_t]),
     "cr_peak_fma": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double),

@@ -646,6 +646,7 @@ struct cr_engine {
     bool uploaded = false, marched = false;
     bool joined = true;  // no stream holds work that the engine's own has not waited for
     cr_stats st{};
+    cr_cluster_stats cl{};
 
     int fail(int code, const char* fmt, ...) {
         char buf[512];
@@ -1527,6 +1528,10 @@ int cr_create(const cr_batch* b, cr_engine** out) {
         for (const auto& g : e->col_groups)
             for (int k = g.begin; k < g.begin + g.count; ++k) e->term_capacity[(size_t)cord[k]] = g.terms;
         e->col_ray = cord;
+        e->cl.rays = (int)cord.size();
+        for (int rid : cord) e->cl.register_rays += lrows[(size_t)rid] > 0;
+        // the refined form has no march on clusters: its rays there run complex128
+        if (e->st.precision_used == CR_C64_REFINED && e->n_tiles == 0) e->st.precision_used = CR_PLAIN_C128;
         e->col_elems = off;
         e->fac_elems = 0;
     } else {
@@ -1837,7 +1842,7 @@ int cr_march(cr_engine* e) {
         ca.compute_grids = e->compute_grids;
         const int chosen = e->precision == CR_CHOSEN_C64R || e->precision == CR_CHOSEN_C64;
         ce = cudaEventRecord(e->ev[0], e->stream);
-        int nl = 0, n_policy = 0;
+        int nl = 0, n_policy = 0, n_reg = 0;
         // column groups first, each on its own stream (they hold the longest
         // marches), then the batched tiles on the engine's stream
         if (ce == cudaSuccess) ce = cudaEventRecord(e->ev_fork, e->stream);
@@ -1853,6 +1858,7 @@ int cr_march(cr_engine* e) {
             if (ce == cudaSuccess) ce = cudaEventRecord(g.done, g.stream);
             ++nl;
             n_policy += g.policy ? 1 : 0;
+            n_reg += g.rows ? 1 : 0;
         }
         sa.tile_begin = 0;
         sa.ticket = e->d_ticket;
@@ -1888,6 +1894,8 @@ int cr_march(cr_engine* e) {
             if (ce == cudaSuccess) ce = cudaStreamWaitEvent(e->stream, g.done, 0);
         e->st.kernel_launches = nl + nb;
         e->st.column_launches = n_policy;
+        e->cl.launches = nl;
+        e->cl.register_launches = n_reg;
     } else if (ce == cudaSuccess) {
         ce = cudaEventRecord(e->ev[0], e->stream);
         if (ce == cudaSuccess) {
@@ -2028,6 +2036,12 @@ int cr_ray_flags(cr_engine* e, int32_t* flags, int n) {
 int cr_get_stats(const cr_engine* e, cr_stats* st) {
     if (!e || !st) return CR_EINVAL;
     *st = e->st;
+    return CR_OK;
+}
+
+int cr_get_cluster_stats(const cr_engine* e, cr_cluster_stats* st) {
+    if (!e || !st) return CR_EINVAL;
+    *st = e->cl;
     return CR_OK;
 }
 

@@ -111,9 +111,12 @@ class Engine:
         return f
 
     def stats(self):
-        st = _lib.CrStats()
+        """cr_stats, and cr_cluster_stats under cluster_rays, cluster_register_rays and so on."""
+        st, cl = _lib.CrStats(), _lib.CrClusterStats()
         _lib.check(self.lib.cr_get_stats(self.handle, ctypes.byref(st)), self.handle)
-        return {k: getattr(st, k) for k, _ in st._fields_}
+        _lib.check(self.lib.cr_get_cluster_stats(self.handle, ctypes.byref(cl)), self.handle)
+        return {**{k: getattr(st, k) for k, _ in st._fields_},
+                **{f"cluster_{k}": getattr(cl, k) for k, _ in cl._fields_}}
 
     def close(self):
         if getattr(self, "handle", None):

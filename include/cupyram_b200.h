@@ -138,14 +138,17 @@ typedef struct cr_stats {
     int64_t device_bytes;     /* device memory held by the engine               */
     int32_t column_rays;      /* rays that the column policy took out of the batch */
     int32_t column_launches;  /* cluster launches of the last cr_march that held
-                                 only such rays; in complex128 the batch's other
-                                 rays march on clusters too                      */
+                                 only such rays.  What marched on clusters, in
+                                 complex128 the batch's other rays among them:
+                                 cr_get_cluster_stats                           */
     int32_t queue_ctas;       /* CTAs of the persistent batched launch (0: none,
                                  or one launch per lanes-per-ray value)        */
     int32_t precision_used;   /* enum cr_precision the march runs in: the
                                  batch's, except that a batch with a source in
                                  the first depth cell (zs < dz) runs the
-                                 complex128 product form in every form         */
+                                 complex128 product form in every form, and a
+                                 refined one whose rays all march on clusters
+                                 runs complex128                               */
     double create_ms;         /* host wall time of cr_create                    */
     double pade_ms;           /* host wall time of the device Pade sets in it   */
     double tuner_row_step_s;  /* measured batched cost the column policy used:
@@ -154,6 +157,18 @@ typedef struct cr_stats {
     double tuner_updates_per_s; /* measured batched throughput it used          */
     double tuner_slots;       /* batched tiles the device holds at once         */
 } cr_stats;
+
+/* What an engine marches on thread-block clusters: laid out by cr_create, and
+ * launched by the last cr_march (0 before one).  The other rays march in
+ * batched tiles (cr_stats.n_tiles of them, kernel_launches - launches
+ * launches). */
+typedef struct cr_cluster_stats {
+    int32_t rays;              /* rays on clusters                               */
+    int32_t register_rays;     /* of these with their factors in registers
+                                  (complex128, columns up to 6144 rows)          */
+    int32_t launches;          /* cluster launches                               */
+    int32_t register_launches; /* of these with factors in registers             */
+} cr_cluster_stats;
 
 typedef struct cr_engine cr_engine;
 
@@ -235,6 +250,8 @@ int cr_set_pade(cr_engine* e, int ray, int which, int n, const double* pd1, cons
 int cr_ray_flags(cr_engine* e, int32_t* flags, int n);
 
 int cr_get_stats(const cr_engine* e, cr_stats* st);
+
+int cr_get_cluster_stats(const cr_engine* e, cr_cluster_stats* st);
 
 /* Copy the last error message (NUL-terminated, truncated to len). */
 int cr_last_error(const cr_engine* e, char* buf, size_t len);
