@@ -278,11 +278,33 @@ def tl_errors(tl_ref, tl):
     return float(d.max()) if d.size else 0.0, float(np.sqrt(np.mean(d * d))) if d.size else 0.0
 
 
-FORM_DESC = {"chosen": "complex64 factors and workspace, FP32 sweeps, FP64 term combination and field",
+FORM_DESC = {"plain": "complex128",
+             "chosen": "complex64 factors and workspace, FP32 sweeps, FP64 term combination and field",
              "fast": "complex64 factors and workspace, FP32 inner loop (sweeps, couplings, M u and term "
                      "combination in FP32); FP64 factorisation and field",
              "refined": "the chosen form plus one iterative-refinement step per Pade term and range step: "
                         "FP64 residual, correction solved with the same complex64 factors (two passes a step)"}
+
+
+def form_marched(form, st):
+    """The form that a march asked for as `form` ran in: refined batches that march on clusters run complex128."""
+    from cupyram_b200 import _lib
+    return "plain" if st["precision_used"] == _lib.CR_PLAIN_C128 else form
+
+
+def roofline(pu, march_s, form, st, peak, traffic_per_update):
+    """Achieved bandwidth on the algorithmic bytes of the form that ran, for pu updates in march_s seconds."""
+    b = B_ALG[form_marched(form, st)]
+    achieved = pu * b / march_s / 1e9
+    tpp = traffic_per_update
+    r = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+         "bytes_per_point_update": b, "traffic": (tpp * pu) if tpp else None,
+         "traffic_gbs": (tpp * pu / march_s / 1e9) if tpp else None,
+         "traffic_frac": (tpp * pu / march_s / 1e9 / peak) if tpp else None}
+    if not st["n_tiles"]:
+        r["note"] = ("every ray marches on a cluster with its column on the chip: these bytes are what a march "
+                     "through memory would move, and do not bound this one")
+    return r
 
 
 def chosen_form(a, batch, out_plain, torch, world, pg, barrier, peak, form="chosen"):
@@ -307,21 +329,16 @@ def chosen_form(a, batch, out_plain, torch, world, pg, barrier, peak, form="chos
         gmax, grms = tl_errors(refs["tlg"], out["tlg"].numpy())
         errs.update(tl_grid_err_max_db=gmax, tl_grid_err_rms_db=grms,
                     tl_grid_cells=int(np.sum(np.isfinite(refs["tlg"]) & (refs["tlg"] < 100.0))))
-    n_tiles = eng.stats()["n_tiles"]
+    st = eng.stats()
     eng.close()
     tll_chosen = out["tll"].numpy().copy()
     pu = batch.point_updates
     value = whole_job_rate(sum_over_ranks(pg, pu), a.steps, t)
-    per_launch_s = float(np.mean(ms)) * 1e-3
-    achieved = pu * B_ALG["chosen"] / per_launch_s / 1e9
-    tpp = profiled_traffic(form, n_tiles) if a.config == "munk" else None
-    return {"form": FORM_DESC[form], "precision": form,
+    tpp = profiled_traffic(form, st["n_tiles"]) if a.config == "munk" else None
+    marched = form_marched(form, st)
+    return {"form": FORM_DESC[marched], "precision": form, "precision_used": marched,
             "value": value, "unit": UNIT, "ms_per_step": t / a.steps, **errs,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "bytes_per_point_update": B_ALG["chosen"],
-                         "traffic": (tpp * pu) if tpp else None,
-                         "traffic_gbs": (tpp * pu / per_launch_s / 1e9) if tpp else None,
-                         "traffic_frac": (tpp * pu / per_launch_s / 1e9 / peak) if tpp else None}}, tll_chosen
+            "roofline": roofline(pu, float(np.mean(ms)) * 1e-3, form, st, peak, tpp)}, tll_chosen
 
 
 def alloc_pinned(batch, torch):
@@ -552,19 +569,13 @@ def main():
             pg.destroy_process_group()
         return 0
     per_launch_s = float(np.mean(march_ms)) * 1e-3
-    achieved = pu * B_ALG[a.form] / per_launch_s / 1e9
     tpp = profiled_traffic(a.form, st["n_tiles"]) if a.config == "munk" else None
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": t_march / a.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "complex128" if a.form == "plain" else "complex64",
+            "dtype": "complex128" if form_marched(a.form, st) == "plain" else "complex64",
             "data": "synthetic", "config": cfg,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "peak_source": peak_kind,
-                         "bytes_per_point_update": B_ALG[a.form],
-                         "traffic": (tpp * pu) if tpp else None,
-                         "traffic_gbs": (tpp * pu / per_launch_s / 1e9) if tpp else None,
-                         "traffic_frac": (tpp * pu / per_launch_s / 1e9 / peak) if tpp else None},
+            "roofline": dict(roofline(pu, per_launch_s, a.form, st, peak, tpp), peak_source=peak_kind),
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d_b),
                     "d2h_bytes_per_step": int(d2h_b),
                     "calls": "cr_create + cr_run (upload, march, download to pinned host buffers) + cr_destroy",
