@@ -50,6 +50,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 
 #include "march_col_math.cuh"
 #include "march_reg.cuh"
@@ -92,6 +93,7 @@ struct RegCtl {
     int per_bt;
     int line_row;            // the line lies between this row and the next,
     double line_dir;         // this far down
+    unsigned idle[CR_MAX_NP];  // steps so far that the term sat out
 };
 constexpr unsigned kCtlBytes = 320;
 static_assert(sizeof(RegCtl) <= kCtlBytes, "RegCtl must fit its slot");
@@ -687,10 +689,10 @@ __device__ __forceinline__ void reg_sum(const ColArgs& a, const RegCtx& x, doubl
 
 // One range step of the active set; out >= 0: the step's field is output
 // `out` (outpt.py:11-57; transmission loss follows at the end, reg_tl).
-// used: steps that this warp's term took part in before.
+// step: index of the step, the self-starter's three included.
 template <int L, bool ALL>
 __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int na, const double2 (&al)[L],
-                                         const double2 (&mw)[L], unsigned used, int out) {
+                                         const double2 (&mw)[L], int step, int out) {
     using O = RegOff<L, ALL>;
     constexpr unsigned P16 = 512u * L;  // bytes of a per-row table
     const int k = x.term, l = x.lane, terms = (int)(blockDim.x >> 5);
@@ -748,6 +750,7 @@ __device__ __forceinline__ void reg_step(const ColArgs& a, const RegCtx& x, int 
         double2 e = shfl2_up(h, 1);
         if (l == 0) e = c2(0.0, 0.0);
         // the mailbox of this step: the two alternate over the term's active steps
+        const unsigned used = (unsigned)step - lds1(sm + O::ctl + (unsigned)offsetof(RegCtl, idle) + 4u * (unsigned)k);
         const unsigned box = used & 1u, par = (used >> 1) & 1u;
         const unsigned to = x.C > 1 ? remote_addr(tm + O::mail + 512u * box + 32u * (unsigned)x.c,
                                                   (unsigned)min(l, x.C - 1)) : 0u;
@@ -983,6 +986,7 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int p = threadIdx.x; p < 32 * L; p += blockDim.x) x.at<double2>(O::U)[p] = c2(0.0, 0.0);
+    if (x.lane == 0) ctl->idle[x.term] = 0u;
     x.own(O::mail)[x.lane] = x.own(O::mail)[32 + x.lane] = c2(0.0, 0.0);
     __syncthreads();
     reg_assemble(a, ctl, 0, ctl->nz + 1);
@@ -1014,7 +1018,6 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
     double2 al[L], mw[L];
     const int steps = a.rays[ctl->rid].nr + 3;
     int na = 0, due = ctl->ndr, tlc = 0, stop;
-    int idle = 0;  // steps so far that this warp's term sat out
 #pragma unroll 1
     for (int s = 0; s < steps; s = stop) {
         int want = s == 0 ? 0 : 1;
@@ -1054,9 +1057,9 @@ __global__ void __maxnreg__(reg_cap<L>()) march_reg_kernel(const __grid_constant
                 if (tlc < ctl->nvr) out = tlc;
                 ++tlc;
             }
-            reg_step<L, ALL>(a, x, na, al, mw, (unsigned)(q - idle), out);
+            reg_step<L, ALL>(a, x, na, al, mw, q, out);
         }
-        if (x.term >= na) idle += stop - s;
+        if (x.term >= na && x.lane == 0) ctl->idle[x.term] += (unsigned)(stop - s);
     }
     if (threadIdx.x == 0 && ctl->dead) atomicOr(a.flags + ctl->rid, 2);
     __threadfence();
