@@ -40,10 +40,14 @@ public:
         return ce;
     }
 
-    // Waits for what still runs on the lane (a microsecond when nothing does).
+    // Waits for what still runs on the lane.
     void give(int dev, StreamLane l) {
         if (!l.stream) return;
-        const bool idle = cudaStreamSynchronize(l.stream) == cudaSuccess;
+        bool idle = cudaStreamQuery(l.stream) == cudaSuccess;
+        if (!idle) {
+            cudaGetLastError();  // the query's "not ready"
+            idle = cudaStreamSynchronize(l.stream) == cudaSuccess;
+        }
         if (idle && dev >= 0 && dev < kDevices) {
             std::lock_guard<std::mutex> lock(mu_);
             if (idle_[dev].size() < kKept) {

@@ -11,7 +11,7 @@
 #include <functional>
 #include <mutex>
 
-enum cudaError_t { cudaSuccess = 0, cudaErrorInvalidDevice = 101 };
+enum cudaError_t { cudaSuccess = 0, cudaErrorInvalidDevice = 101, cudaErrorNotReady = 600 };
 enum cudaMemcpyKind { cudaMemcpyHostToDevice, cudaMemcpyDeviceToHost };
 constexpr unsigned cudaHostAllocPortable = 1, cudaEventDisableTiming = 2, cudaStreamNonBlocking = 1;
 
@@ -90,6 +90,12 @@ inline cudaError_t cudaEventSynchronize(cudaEvent_t e) {
     while (e->stream && !e->stream->work.empty()) fake::run(e->stream, 1);
     return cudaSuccess;
 }
+inline cudaError_t cudaStreamQuery(cudaStream_t s) {
+    FAKE_LOCK;
+    fake::check(s->device);
+    return s->work.empty() ? cudaSuccess : cudaErrorNotReady;
+}
+inline cudaError_t cudaGetLastError() { return cudaSuccess; }
 inline cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     FAKE_LOCK;
     fake::check(s->device);
