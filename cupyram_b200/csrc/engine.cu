@@ -1247,9 +1247,12 @@ int reg_active(int device, int cluster, int terms, int rows, int grids) {
 }
 
 // Microseconds of one step of march_reg.cu with `rows` rows a lane, with the
-// SMs' other CTAs at work.  B200, np 6: 2.3 / 2.7 / 3.1 / 3.5 / 4.9 us at 4 / 6 /
-// 8 / 10 / 12 rows on single CTAs; 0.5 us more on pairs, 0.8 us more on
-// clusters of 16 (the exchange).
+// SMs' other CTAs at work.  The line is that of the first kernels (B200, np 6, single
+// CTAs: 2.3 / 2.7 / 3.1 / 3.5 / 4.9 us at 4 / 6 / 8 / 10 / 12 rows; 0.5 us more on
+// pairs, 0.8 us more on clusters of 16, the exchange).  Those of today take 1.9 / 2.2 /
+// 2.6 / 3.1 / 3.9 us, 2.6 / 2.7 / 3.3 at 7 / 9 / 11 rows, pairs 3.2 / 3.7 / 4.6 at 8 /
+// 10 / 12, clusters of 16 4.5 / 4.8 at 11 / 12: the line is 0.2 to 1.4 us high, most at
+// 11 rows.  Only its ratios between shapes enter the plan.
 double reg_step_us(int cluster, int rows) {
     const double t = 1.55 + 0.19 * rows + (rows > 10 ? 1.0 : 0.0);
     return cluster == 1 ? t : t + 0.4 + 0.1 * std::log2((double)cluster);
@@ -1258,15 +1261,16 @@ double reg_step_us(int cluster, int rows) {
 // Cluster and rows of a lane of the rays that march_reg.cu takes: in complex128,
 // every ray whose column fits the registers of at most 16 CTAs.  Against the
 // batched kernel (72-78e9 term-rows per second at any depth, bound by its
-// streams from memory) it marched 123e9 on one CTA of 380 rows, 107e9 on two,
-// 104e9 at 2300 and 3800 rows and 82e9 at 5300 - 5700 rows (16 CTAs of 11 or 12
-// rows a lane; of 12 alone: 78e9).
+// streams from memory) it marches 175e9 on one CTA of 380 rows, 142-156e9 on pairs,
+// 120-123e9 at 2300 and 3800 rows and 100-102e9 at 5300 - 5700 rows (np 6, flat
+// bottoms, batches that fill the GPU).
 //
 // The cluster of a ray is the one that minimises the larger of its own march
 // and the whole batch's at that shape's throughput: long rays of an uneven
-// batch get many CTAs and short steps, the others few and full lanes.  Up to
-// nine rays have the GPU to themselves: they get what march_col.cu would give
-// them (as many CTAs as there are SMs, at least 64 rows each).
+// batch get many CTAs and short steps, the others few and full lanes.  Operator
+// changes are not counted.  Up to nine rays have the GPU to themselves: they get
+// what march_col.cu would give them (as many CTAs as there are SMs, at least 64
+// rows each; the line at nine rays is that kernel's and was not measured for this one).
 struct RegPlan {
     int cluster = 0, rows = 0;
 };
@@ -1921,7 +1925,7 @@ int cr_march(cr_engine* e) {
     e->st.rays_failed = failed;
     e->marched = true;
     if (timed_out)
-        return e->fail(CR_ETIMEOUT, "%d ray(s): a wait for the march's bulk copies gave up", timed_out);
+        return e->fail(CR_ETIMEOUT, "%d ray(s): a bounded wait of the march (bulk copies or mailboxes) gave up", timed_out);
     if (failed) return e->fail(CR_ENAN, "%d ray(s) produced a non-finite field", failed);
     return CR_OK;
 }

@@ -6,16 +6,21 @@
 //     forward        Y[B,N]  = X[B,K]  W[N,K]^T            (+ bias, ReLU)
 //     input grad     dX[B,K] = dY[B,N] (W^T)[K,N]^T         (x ReLU mask)
 //     weight grad    dW[N,K] = (dY^T)[N,B] (X^T)[K,B]^T
-// with transposed BF16 copies of W, dY and X made by a tiled transpose.  The
-// tile loop stages 128 x 32 tiles of A and B in shared memory with cp.async
-// (two stages, XOR-swizzled 16-byte chunks so that ldmatrix reads are
-// conflict-free), and each of 8 warps runs mma.sync m16n8k16 (bf16 x bf16 ->
-// f32) on a 64 x 32 piece of the 128 x 128 block.  Shapes must be multiples of
-// the tile (M, N of 128, K of 32); the host wrappers check that and the
-// 16-byte alignment of every row.
+// with transposed BF16 copies of W, dY and X made by a tiled transpose.
 //
-// The same contraction also runs on the 5th-generation tensor cores
-// (gemm_tn_umma: tcgen05.mma with the accumulator in tensor memory).
+// Shapes with N a multiple of 256 and K of 64 run on the 5th-generation tensor
+// cores (tcgen05.mma, accumulators in tensor memory, operands and results moved
+// by the tensor memory accelerator): gemm_tn_tile, gemm_tn_persistent for large
+// outputs, ensemble_tile for an ensemble's output layers.  gemm_tn_tma takes
+// outputs and masks whose rows do not start on 16-byte boundaries, gemm_tn_umma
+// (operands by cp.async) stands behind CUPYRAM_B200_GEMM=cp.
+//
+// Other shapes run on gemm_tn: 128 x 32 tiles of A and B staged in shared memory
+// with cp.async (two stages, XOR-swizzled 16-byte chunks so that ldmatrix reads
+// are conflict-free), each of 8 warps running mma.sync m16n8k16 (bf16 x bf16 ->
+// f32) on a 64 x 32 piece of the 128 x 128 block.  Shapes must be multiples of
+// the tile (M, N of 128, K of 32); the host wrappers check that and the 16-byte
+// alignment of every row.
 //
 // Plus the small kernels of a training step: column sums (bias gradients),
 // the masked mean-squared-error gradient, Adam, and BF16 conversion.
@@ -216,7 +221,7 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
     d |= (uint64_t)2 << 61;                // SWIZZLE_128B
     return d;
 }
-// Instruction descriptor: D f32, A and B bf16, both K-major, M 128, N 128.
+// Instruction descriptor: D f32, A and B bf16, both K-major, M 128, N 256.
 constexpr uint32_t kUIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(UBN >> 3) << 17) | ((uint32_t)(UBM >> 4) << 24);
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
@@ -673,7 +678,9 @@ __device__ __forceinline__ void store_sector(void* p, const uint32_t* w) {
 }
 
 // Kernels launched by launch_next start beside the end of the one before: what a
-// CTA sets up for itself - tensor memory, barriers - overlaps it.  Nothing of global
+// CTA sets up for itself - tensor memory, barriers - overlaps it (shared memory admits
+// two CTAs of gemm_tn_tile on an SM, or one of any other tcgen05 kernel that waits here, so
+// its 512 columns never run short).  Nothing of global
 // memory is read or written before this returns, which is when that kernel has
 // completed; the next launch may then start in the same way.  (Not for kernels whose
 // inputs are const __restrict__: such loads may be moved above the wait.)  A training step of 512
@@ -840,9 +847,6 @@ __device__ __forceinline__ int mat_of(const Mats& t, int block) {
     return i;
 }
 
-// dst[c][r] = src[r][c] in 64 x 64 tiles: 16-byte rows in and out (columns and
-// rows multiples of 64, bases and strides 16-byte aligned).  All layers of a
-// training step in one launch, instead of twelve of 3.5-11 us.
 // Place of (c, r) in row c of a transposed 64 x 64 tile: the 16-byte pieces of a row
 // are permuted by the row's eighth, or the lanes of a warp, eight columns apart,
 // would write one bank (with the column sums' eight loads in flight, a training step
@@ -855,6 +859,9 @@ struct __align__(16) Tile64 {
 };
 static_assert(alignof(Tile64) >= 16 && sizeof(Tile64) % (64 * 16) == 0, "rows on 16-byte boundaries");
 
+// dst[c][r] = src[r][c] in 64 x 64 tiles: 16-byte rows in and out (columns and
+// rows multiples of 64, bases and strides 16-byte aligned).  All layers of a
+// training step in one launch, instead of twelve of 3.5-11 us.
 __global__ void __launch_bounds__(256) transpose_mats(const __grid_constant__ Mats t) {
     __shared__ Tile64 tile;
     const int i = mat_of(t, blockIdx.x), b = blockIdx.x - t.first[i], nc = t.cols[i] / 64;
@@ -1115,10 +1122,11 @@ int grid_for(long long n) {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// The kernel behind cr_mlp_gemm_tc: the TMA-fed one, one block per CTA and
-// two CTAs per SM, by default (measured fastest: 515 TFLOP/s on 8192 x 8192 x
-// 512, against 392 for the persistent one and 480 for the cp.async-fed one);
-// CUPYRAM_B200_GEMM=persistent the persistent one, =cp the cp.async-fed one.
+// How cr_mlp_gemm_tc feeds its kernels: 1, the default, by the tensor memory
+// accelerator (launch_tile_n chooses among gemm_tn_tile's blocks and
+// gemm_tn_persistent; gemm_tn_tma for rows off 16-byte boundaries);
+// CUPYRAM_B200_GEMM=persistent: gemm_tn_persistent at any size, =cp: gemm_tn_umma,
+// fed by cp.async.
 int gemm_feed() {
     const char* v = getenv("CUPYRAM_B200_GEMM");
     if (v && v[0] == 'c') return 0;
@@ -1127,13 +1135,14 @@ int gemm_feed() {
 }
 
 // ---------------------------------------------------------------------------
-// Persistent contraction with the epilogue overlapped, for outputs of many
-// blocks.
+// Persistent contraction with the epilogue overlapped, for outputs of at least
+// two blocks an SM.
 //
 // One CTA per SM walks the output blocks (128 x 256) in a static round
 // robin.  Six warps:
-//   * warp 0, lane 0: TMA producer over a kPStages-deep ring of stages;
-//   * warp 1, lane 0: MMA issuer, accumulating block i in one of two TMEM
+//   * warp 0: TMA producer over a kPStages-deep ring of stages (one elected lane
+//     issues, as in gemm_tn_tile);
+//   * warp 1: MMA issuer, accumulating block i in one of two TMEM
 //     accumulators (columns 0..255 or 256..511, by i's parity), committing
 //     each stage to its "empty" barrier and each finished block to its
 //     accumulator's "full" barrier;
@@ -1584,21 +1593,19 @@ bool aligned32(const void* p) { return ((uintptr_t)p & 31) == 0; }
 // kernel at any size (a mask takes its shared memory: never there).
 template <int EPI>
 cudaError_t launch_tile_n(const TileOperands& o, const EpiArgs& e, bool walk, int* err, cudaStream_t st) {
-    constexpr int kSms = 148;
-    const long long rows = o.M / UBM;
+    const long long rows = o.M / UBM, sms = sm_count();
     if constexpr (EPI != CR_MLP_EPI_RELU_MASK_BF16) {
-        if (walk || rows * (o.N / 256) >= 2 * kSms) return launch_persistent<EPI>(o, e, err, st);
+        if (walk || rows * (o.N / 256) >= 2 * sms) return launch_persistent<EPI>(o, e, err, st);
     }
-    if (rows * (o.N / 128) >= kSms) return launch_tile<EPI, 128, 3, 1>(&o, &e, err, st);
+    if (rows * (o.N / 128) >= sms) return launch_tile<EPI, 128, 3, 1>(&o, &e, err, st);
     return launch_tile<EPI, 64, 7, 1>(&o, &e, err, st);
 }
 
 // G equal hidden layers (bias, ReLU, bf16) in one launch.
 template <int G>
 cudaError_t launch_hidden(const TileOperands* o, const EpiArgs* e, int* err, cudaStream_t st) {
-    constexpr int kSms = 148;
     const long long rows = (long long)(o[0].M / UBM) * G;
-    if (rows * (o[0].N / 128) >= kSms) return launch_tile<CR_MLP_EPI_BIAS_RELU_BF16, 128, 3, G>(o, e, err, st);
+    if (rows * (o[0].N / 128) >= sm_count()) return launch_tile<CR_MLP_EPI_BIAS_RELU_BF16, 128, 3, G>(o, e, err, st);
     return launch_tile<CR_MLP_EPI_BIAS_RELU_BF16, 64, 7, G>(o, e, err, st);
 }
 

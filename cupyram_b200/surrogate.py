@@ -12,10 +12,12 @@ the march.  PyTorch only holds device buffers and streams.
 
 Training fields and fallback fields come from the march's chosen form
 (complex64 sweeps; <= 0.01 dB RMS from complex128 on every measured
-workload, far below the network's own error), whose half-size shared
-footprint lets the column-parallel kernel take the deep, high-frequency
-columns of this distribution.  The judge reruns use the plain complex128
-march.
+workload, far below the network's own error).  It was chosen when complex128
+needed twice the shared memory for the deep, high-frequency columns of this
+distribution; complex128 has since moved to registers and is the faster one on
+uneven batches (10,000 wedge rays 3.6 s against 8.7-9.4 s), but the fields'
+form stays what the trained members were measured with.  The reruns that
+judge served fields use plain complex128.
 
 Coarse field.  Cell (i, j) covers ranges (i, i+1] x 156.25 m and depths
 (j, j+1] x D0 / 64 (D0: water depth at the source).  Its TL is
