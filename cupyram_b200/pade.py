@@ -26,7 +26,7 @@ def compute_pade_coefficients(freq, c0, np_pade, ns=1, dr=50.0, ip=1):
 
 def pade_batch(freq, c0, np_pade, ns, dr, ip):
     """Pade coefficients of many jobs at once, solved on the current CUDA device
-    (cr_pade_batch, one thread per job, the same FP64 construction as
+    (cr_pade_batch, one warp per job, the same FP64 construction as
     :func:`compute_pade_coefficients`).  Every argument is a scalar or an array
     broadcast to the batch.  Returns ``(pd1, pd2, status)``: complex128
     ``[n, CR_MAX_NP]`` arrays (zeros past each job's np) and the per-job
